@@ -165,6 +165,31 @@ int lens_te2d_step_driven(const LensTE2D *g, const LensStepTable *tab, const Len
 int lens_tm2d_step_driven(const LensTM2D *g, const LensStepTable *tab, const LensEpi2D *ep,
                           const LensDrive2D *drive, int n0, int nsteps, void *stream);
 
+/* The same steps in ONE cooperative launch that keeps the fields in registers, for a
+ * grid whose state fits on the chip (ny <= 768, at most 20 rows per band and one band or
+ * more per SM): bands of x rows exchange one row per step through L2.  Fields, psi and
+ * sums hold the bits that lens_te2d_step / lens_tm2d_step would leave (FP64 sums of boxes
+ * and planes to their last digits), so a caller may mix the two.  *_bytes: device scratch
+ * the launch needs, 0 when the grid does not fit.  A call that the resident launch does
+ * not carry (the epilogue's dft_raw, ex2 or nsx planes, a capturing stream, nsteps < 1,
+ * too little scratch) returns LENS_ERR_SIZE before anything is enqueued: step it with
+ * the entries above.  The call zeroes scratch on `stream`.  Waits between bands are
+ * bounded (seconds at most); if one runs out *err (a device int, zeroed once by the
+ * caller) becomes nonzero, the launch ends and the band's fields become NaN.  The
+ * launch takes every SM it plans for.                                         */
+size_t lens_te2d_resident_bytes(const LensTE2D *g);
+size_t lens_tm2d_resident_bytes(const LensTM2D *g);
+int lens_te2d_resident(const LensTE2D *g, const LensStepTable *tab, const LensEpi2D *ep, int n0, int nsteps,
+                       void *scratch, size_t bytes, int *err, void *stream);
+int lens_tm2d_resident(const LensTM2D *g, const LensStepTable *tab, const LensEpi2D *ep, int n0, int nsteps,
+                       void *scratch, size_t bytes, int *err, void *stream);
+
+/* Watchdog self-test (no counterpart in the reference): the launch with every wait cut
+ * to 1024 polls and the second band withholding its first E row of step 1; *err becomes
+ * nonzero, every band leaves its step loop.  Needs two bands and nsteps >= 3.   */
+int lens_te2d_resident_watchdog_test(const LensTE2D *g, const LensStepTable *tab, int n0, int nsteps, void *scratch,
+                                     size_t bytes, int *err, void *stream);
+
 /* ------------------------------------------------------- batched 2D solves
  * Many independent 2D solves of uneven sizes (TE and TM mixed) advanced together:
  * one launch per half step covers every tile of every instance, so a sweep of

@@ -86,6 +86,7 @@ class Epi3D(ctypes.Structure):
                 ('nplane', c_int), ('plane', c_int * MAX_PLANE), ('plane_acc', c_void_p)]
 
 
+ERR_SIZE = -3               # LENS_ERR_SIZE
 F32, F16, BF16 = 0, 1, 2   # LENS_F32 / LENS_F16 / LENS_BF16 field storage
 
 
@@ -163,6 +164,14 @@ SIGNATURES = {
                               c_void_p, ctypes.c_size_t, c_void_p, c_void_p]),
     'lens_rs2d_watchdog_test': (c_int, [POINTER(Inst2D), c_void_p, c_int, POINTER(StepTable), c_int, c_int,
                                         c_void_p, ctypes.c_size_t, c_void_p, c_void_p]),
+    'lens_te2d_resident_bytes': (ctypes.c_size_t, [POINTER(TE2D)]),
+    'lens_tm2d_resident_bytes': (ctypes.c_size_t, [POINTER(TM2D)]),
+    'lens_te2d_resident': (c_int, [POINTER(TE2D), POINTER(StepTable), POINTER(Epi2D), c_int, c_int, c_void_p,
+                                   ctypes.c_size_t, c_void_p, c_void_p]),
+    'lens_tm2d_resident': (c_int, [POINTER(TM2D), POINTER(StepTable), POINTER(Epi2D), c_int, c_int, c_void_p,
+                                   ctypes.c_size_t, c_void_p, c_void_p]),
+    'lens_te2d_resident_watchdog_test': (c_int, [POINTER(TE2D), POINTER(StepTable), c_int, c_int, c_void_p,
+                                                 ctypes.c_size_t, c_void_p, c_void_p]),
     'lens_version': (c_int, []),
     'lens_status_string': (ctypes.c_char_p, [c_int]),
     'lens_abi_sizes': (c_int, [POINTER(c_int), c_int]),

@@ -62,6 +62,11 @@ def strip_widths(c):
     return lo, hi
 
 
+# Steps from which Grid2D.step takes the resident launch: a launch of few steps pays for
+# the state's way in and out (see the launch in csrc/grid2d_resident.cuh).
+RS_MIN_STEPS = 4
+
+
 class _Axis:
     """Device copy of one CPML axis (b, c, 1/kappa on integer and half nodes).
     full: psi over the whole axis (every node a strip node: b = 1, c = 0 keeps
@@ -179,6 +184,12 @@ class Grid2D:
                             _ptr(self.psi['hzx']), _ptr(self.psi['hzy']), _ptr(self.psi['exy']),
                             _ptr(self.psi['eyx']), pec4, s)
 
+        # scratch and error word of the resident launch (lens_te2d_resident), when the grid fits the chip
+        need = (self.lib.lens_te2d_resident_bytes if self.pol == 's' else self.lib.lens_tm2d_resident_bytes)(
+            ctypes.byref(self.s))
+        self.rs_scratch = torch.empty(need, dtype=torch.uint8, device=dev) if need else None
+        self.rs_err = torch.zeros(1, dtype=torch.int32, device=dev) if need else None
+
     # reference-shaped views of the resident fields
     def view(self, name):
         nx, ny = self.nx, self.ny
@@ -204,6 +215,12 @@ class Grid2D:
 
     def step(self, table, n0, nsteps, epi=None, stream=None, drive=None):
         e = ctypes.byref(epi.s) if epi is not None else None
+        if drive is None and self.rs_scratch is not None and nsteps >= RS_MIN_STEPS:
+            fn = self.lib.lens_te2d_resident if self.pol == 's' else self.lib.lens_tm2d_resident
+            st = fn(ctypes.byref(self.s), ctypes.byref(table.s), e, int(n0), int(nsteps), _ptr(self.rs_scratch),
+                    self.rs_scratch.numel(), _ptr(self.rs_err), _stream_ptr(stream))
+            if st != N.ERR_SIZE:      # else: a call that only the steps below carry
+                return N.check(st)
         if drive is None:
             fn = self.lib.lens_te2d_step if self.pol == 's' else self.lib.lens_tm2d_step
             N.check(fn(ctypes.byref(self.s), ctypes.byref(table.s), e, int(n0), int(nsteps), _stream_ptr(stream)))
@@ -211,6 +228,12 @@ class Grid2D:
             fn = self.lib.lens_te2d_step_driven if self.pol == 's' else self.lib.lens_tm2d_step_driven
             N.check(fn(ctypes.byref(self.s), ctypes.byref(table.s), e, ctypes.byref(drive.s), int(n0),
                        int(nsteps), _stream_ptr(stream)))
+
+
+    def check(self):
+        """Raise if a resident launch's wait between bands ran out (the fields hold NaN then)."""
+        if self.rs_err is not None and int(self.rs_err.item()) != 0:
+            raise N.LensError('resident 2D launch: a wait between bands timed out (results invalid)')
 
 
 class Drive2D:
