@@ -688,128 +688,138 @@ __device__ __forceinline__ unsigned epi_parts(const LensEpi2D &ep, int n) {
            (ep.dft_prev && n >= ep.prev_n0 && n < ep.prev_n1 ? EP_PREV : 0u) | (ep.iavg && n >= ep.iavg_n0 ? EP_IAVG : 0u);
 }
 
-// Compensated complex sum (lens_common.cuh's kahan_add, its first product fused as there).
-__device__ __forceinline__ void kahan_fma(float4 &a, float v, float pr, float pim) {
-    float y = __fmaf_rn(v, pr, -a.z), t = __fadd_rn(a.x, y);
-    a.z = __fsub_rn(__fsub_rn(t, a.x), y);
-    a.x = t;
-    y = __fmaf_rn(v, pim, -a.w);
-    t = __fadd_rn(a.y, y);
-    a.w = __fsub_rn(__fsub_rn(t, a.y), y);
-    a.y = t;
+// Compensated complex sum (lens_common.cuh's kahan_add, its first product fused as
+// there), real and imaginary part at once: a = (sum, carry), np = minus the phase.
+// With m = carry - v phase = -y, the sum is t = sum - m and the carry (t - sum) + m.
+__device__ __forceinline__ void kahan_pair(float4 &a, float v, float2 np) {
+    const float2 s = make_float2(a.x, a.y), m = fma2(f2(v), np, make_float2(a.z, a.w)), t = sub2(s, m);
+    const float2 c = __fadd2_rn(sub2(t, s), m);
+    a = make_float4(t.x, t.y, c.x, c.y);
 }
 
 // Rows whose sums travel together.
-constexpr int EPI_G = 2;
+constexpr int EPI_G = 4;
 
-// Compensated sums of the rows r0 .. r0+G-1 of a thread's two columns; d: the thread's
-// first row in a (node, 4 floats) array of row pitch P nodes.
-template <int RM>
-__device__ __forceinline__ void epi_dft(float *d, size_t P, int r0, int R, bool on1, float pr, float pim,
-                                        const float2 (&v)[EPI_G]) {
-    float4 s[2 * EPI_G];
-#pragma unroll
-    for (int q = 0; q < EPI_G; ++q)
-        if (r0 + q < RM && r0 + q < R) {
-            const float4 *p = reinterpret_cast<const float4 *>(d) + (size_t)(r0 + q) * P;
-            s[2 * q] = p[0];
-            if (on1) s[2 * q + 1] = p[1];
-        }
-#pragma unroll
-    for (int q = 0; q < EPI_G; ++q)
-        if (r0 + q < RM && r0 + q < R) {
-            float4 *p = reinterpret_cast<float4 *>(d) + (size_t)(r0 + q) * P;
-            kahan_fma(s[2 * q], v[q].x, pr, pim);
-            p[0] = s[2 * q];
-            if (on1) {
-                kahan_fma(s[2 * q + 1], v[q].y, pr, pim);
-                p[1] = s[2 * q + 1];
-            }
-        }
+// Node value of row r: 0 the driven field, 1 (TM) Ex on the nodes, 2 the intensity
+// (fdtd2d_core.py:458-486).  y: TM, the Ey of the column before each warp's first.
+// Rows at an x face are the general form's, columns at a y face the V_Y form's.
+template <int RM, int POL, unsigned V>
+__device__ __forceinline__ float2 node_value(const Th<RM> &t, const Band &B, int r, int what, float y) {
+    if (POL == 0) return what == 2 ? mul2(t.a[r], t.a[r]) : t.a[r];
+    const float2 ey = t.b[r], lo = pair_dn(ey, t.lane, y);
+    float2 F = mul2(f2(0.5f), make_float2(lo.x + ey.x, lo.y + ey.y));
+    if (V & V_Y) {
+        const int j = t.w * 64 + 2 * t.lane, ny = B.ny;
+        F.x = j == 0 ? ey.x : (j == ny - 1 ? lo.x : F.x);
+        F.y = j + 1 == ny - 1 ? lo.y : F.y;
+    }
+    if (what == 0) return F;
+    const float2 p = r > 0 ? t.a[r > 0 ? r - 1 : 0] : t.ga, c = t.a[r];  // Ex of rows i-1 and i
+    float2 X = mul2(f2(0.5f), make_float2(p.x + c.x, p.y + c.y)), s2 = mul2(f2(0.5f), fma2(p, p, mul2(c, c)));
+    if (V & V_X) {
+        const int i = B.lo + r;
+        const bool first = i == 0, last = i == B.nx - 1;
+        const float2 e = sel2(last, last, p, c);
+        X = sel2(first || last, first || last, e, X);
+        s2 = sel2(first || last, first || last, mul2(e, e), s2);
+    }
+    const float2 I = fma2(F, F, s2);
+    return sel2(what == 1, what == 1, X, I);
 }
 
-// The epilogue of one step on a thread's cells.  y: TM, the Ey of the column before
-// each warp's first (edge_in); box: this band meets a detector box.
-template <int RM, int POL>
+// The epilogue of one step on a thread's cells.  box: this band meets a detector box.
+// Loops over the sums stay loops: unrolled for every sum, box and row the code ran from
+// beyond the instruction caches in each of the four row forms and cost 4.8 us a step
+// whatever it had to do.
+template <int RM, int POL, unsigned V>
 __device__ __forceinline__ void epilogue(const Th<RM> &t, const Band &B, const LensEpi2D &ep, const LensStepTable &tab,
                                          int k, unsigned parts, bool box, const float (&y)[rs_edge(RM)], bool hold,
                                          float *sdft, double *bacc) {
     const int j = t.w * 64 + 2 * t.lane, ny = B.ny;
-    const bool on0 = j < ny, on1 = j + 1 < ny;
+    const bool on0 = !(V & V_Y) || j < ny, on1 = !(V & V_Y) || j + 1 < ny;
     const size_t o = (size_t)B.lo * B.P + j;
-    const float pr = (parts & (EP_DFT | EP_EX | EP_PREV)) ? __ldg(tab.pe + 2 * k) : 0.f;
-    const float pim = (parts & (EP_DFT | EP_EX | EP_PREV)) ? __ldg(tab.pe + 2 * k + 1) : 0.f;
-    double bs[LENS_MAX_BOX] = {0.0, 0.0, 0.0, 0.0};
+    if (parts & (EP_DFT | EP_EX | EP_PREV)) {
+        const float2 np = make_float2(-__ldg(tab.pe + 2 * k), -__ldg(tab.pe + 2 * k + 1));
+#pragma unroll 1
+        for (int a = 0; a < (POL == 1 ? 3 : 2); ++a) {  // compensated sums: DFT, comparison window, TM Ex
+            if (!(parts & (a == 0 ? EP_DFT : (a == 1 ? EP_PREV : EP_EX)))) continue;
+            float4 *d = reinterpret_cast<float4 *>(a == 0 ? ep.dft : (a == 1 ? ep.dft_prev : ep.dft_ex)) + o;
+            int P = B.P;
+            if (a == 0 && hold) {
+                d = reinterpret_cast<float4 *>(sdft);
+                P = t.NS;
+            }
 #pragma unroll
-    for (int r0 = 0; r0 < RM; r0 += EPI_G) {
-        float2 F[EPI_G], I[EPI_G], X[EPI_G];
+            for (int r0 = 0; r0 < RM; r0 += EPI_G) {
+                float4 s[2 * EPI_G];
 #pragma unroll
-        for (int q = 0; q < EPI_G; ++q) {
-            const int r = r0 + q < RM ? r0 + q : 0, i = B.lo + r;
-            if (POL == 0) {
-                F[q] = t.a[r];
-                I[q] = mul2(F[q], F[q]);
-                X[q] = f2(0.f);
-            } else {
-                // Ey on the nodes, Ex and its square averaged over rows i-1 and i (fdtd2d_core.py:458-486)
-                const float2 ey = t.b[r], lo = pair_dn(ey, t.lane, y[r]);
-                F[q].x = j == 0 ? ey.x : (j == ny - 1 ? lo.x : 0.5f * (lo.x + ey.x));
-                F[q].y = j + 1 == ny - 1 ? lo.y : 0.5f * (lo.y + ey.y);
-                const float2 p = r > 0 ? t.a[r > 0 ? r - 1 : 0] : t.ga, c = t.a[r];
-                const bool first = i == 0, last = i == B.nx - 1;
-                const float2 e = sel2(last, last, p, c);
-                const float2 in = mul2(f2(0.5f), fma2(p, p, mul2(c, c))), fc = mul2(e, e);
-                const float2 s2 = sel2(first || last, first || last, fc, in);
-                X[q] = sel2(first || last, first || last, e, mul2(f2(0.5f), make_float2(p.x + c.x, p.y + c.y)));
-                I[q] = fma2(F[q], F[q], s2);
+                for (int q = 0; q < EPI_G; ++q)
+                    if (r0 + q < RM && r0 + q < t.R) {
+                        if (on0) s[2 * q] = d[(size_t)(r0 + q) * P];
+                        if (on1) s[2 * q + 1] = d[(size_t)(r0 + q) * P + 1];
+                    }
+#pragma unroll
+                for (int q = 0; q < EPI_G; ++q) {
+                    const int r = r0 + q < RM ? r0 + q : 0;
+                    if (r0 + q >= RM) continue;
+                    const float2 v = node_value<RM, POL, V>(t, B, r, a == 2 ? 1 : 0, y[r]);
+                    if (r >= t.R) continue;
+                    kahan_pair(s[2 * q], v.x, np);
+                    kahan_pair(s[2 * q + 1], v.y, np);
+                    if (on0) d[(size_t)r * P] = s[2 * q];
+                    if (on1) d[(size_t)r * P + 1] = s[2 * q + 1];
+                }
             }
         }
-        if (box)
+    }
+    if (parts & EP_IAVG) {
+        float *a = ep.iavg + o;
 #pragma unroll
-            for (int b = 0; b < LENS_MAX_BOX; ++b)
-                if (b < ep.nbox) {
-                    const int *bx = ep.box[b];
-#pragma unroll
-                    for (int q = 0; q < EPI_G; ++q) {
-                        const int r = r0 + q, i = B.lo + r;
-                        if (r < RM && r < t.R && i >= bx[0] && i < bx[1]) {
-                            if (on0 && j >= bx[2] && j < bx[3]) bs[b] += (double)I[q].x;
-                            if (on1 && j + 1 >= bx[2] && j + 1 < bx[3]) bs[b] += (double)I[q].y;
-                        }
-                    }
-                }
-        if (!on0) continue;
-        if (parts & EP_DFT) {
-            if (hold) epi_dft<RM>(sdft, t.NS, r0, t.R, on1, pr, pim, F);
-            else epi_dft<RM>(ep.dft + 4 * o, B.P, r0, t.R, on1, pr, pim, F);
-        }
-        if (POL == 1 && (parts & EP_EX)) epi_dft<RM>(ep.dft_ex + 4 * o, B.P, r0, t.R, on1, pr, pim, X);
-        if (parts & EP_PREV) epi_dft<RM>(ep.dft_prev + 4 * o, B.P, r0, t.R, on1, pr, pim, F);
-        if (parts & EP_IAVG) {
-            float *a = ep.iavg + o;
+        for (int r0 = 0; r0 < RM; r0 += EPI_G) {
             float2 s[EPI_G];
 #pragma unroll
             for (int q = 0; q < EPI_G; ++q)
-                if (r0 + q < RM && r0 + q < t.R) s[q] = in2(a + (size_t)(r0 + q) * B.P);
-#pragma unroll
-            for (int q = 0; q < EPI_G; ++q)
                 if (r0 + q < RM && r0 + q < t.R) {
-                    a[(size_t)(r0 + q) * B.P] = __fadd_rn(s[q].x, I[q].x);
-                    if (on1) a[(size_t)(r0 + q) * B.P + 1] = __fadd_rn(s[q].y, I[q].y);
+                    if (on0) s[q].x = a[(size_t)(r0 + q) * B.P];
+                    if (on1) s[q].y = a[(size_t)(r0 + q) * B.P + 1];
                 }
+#pragma unroll
+            for (int q = 0; q < EPI_G; ++q) {
+                const int r = r0 + q < RM ? r0 + q : 0;
+                if (r0 + q >= RM) continue;
+                const float2 I = node_value<RM, POL, V>(t, B, r, 2, y[r]);
+                if (r >= t.R) continue;
+                if (on0) a[(size_t)r * B.P] = __fadd_rn(s[q].x, I.x);
+                if (on1) a[(size_t)r * B.P + 1] = __fadd_rn(s[q].y, I.y);
+            }
         }
     }
-    if (box)
+    if (box) {
+#pragma unroll 1
+        for (int b = 0; b < ep.nbox; ++b) {
+            const int lo = ep.box[b][0] - B.lo, hi = min(ep.box[b][1] - B.lo, t.R);
+            const bool c0 = on0 && j >= ep.box[b][2] && j < ep.box[b][3],
+                       c1 = on1 && j + 1 >= ep.box[b][2] && j + 1 < ep.box[b][3];
+            if (hi <= lo || hi <= 0 || !__any_sync(FULL, c0 || c1)) continue;
+            double v[4] = {0.0, 0.0, 0.0, 0.0};  // four chains of FP64 additions
 #pragma unroll
-        for (int b = 0; b < LENS_MAX_BOX; ++b)
-            if (b < ep.nbox) bacc[b * 32 * blockDim.y] += bs[b];
+            for (int r = 0; r < RM; ++r) {
+                const float2 I = node_value<RM, POL, V>(t, B, r, 2, y[r]);
+                const bool in = r >= lo && r < hi;
+                v[r % 2 * 2] += (double)(in && c0 ? I.x : 0.f);
+                v[r % 2 * 2 + 1] += (double)(in && c1 ? I.y : 0.f);
+            }
+            bacc[b * 32 * blockDim.y] += (v[0] + v[1]) + (v[2] + v[3]);
+        }
+    }
     if (parts & EP_PLANE) {
         // Poynting plane DFTs (flux.py:28-41): E on the plane, H averaged over rows il-1 and il
-        const double er = __ldg(tab.pe + 2 * k), ei = __ldg(tab.pe + 2 * k + 1), hr = __ldg(tab.ph + 2 * k),
-                     hi = __ldg(tab.ph + 2 * k + 1);
+#pragma unroll 1
         for (int p = 0; p < ep.nplane; ++p) {
             const int rr = ep.plane[p] - B.lo;
             if (rr < 0 || rr >= t.R) continue;
+            const double er = __ldg(tab.pe + 2 * k), ei = __ldg(tab.pe + 2 * k + 1), hr = __ldg(tab.ph + 2 * k),
+                         hi = __ldg(tab.ph + 2 * k + 1);
             float2 e = f2(0.f), h = f2(0.f), hm = t.gc;
 #pragma unroll
             for (int r = 0; r < RM; ++r) {
@@ -888,7 +898,7 @@ __device__ __forceinline__ bool rs_loop(Th<RM> &t, const Band &B, const GPlan &p
         if (parts || box) {
             float y[EP];
             if (POL == 1) edge_in<RM>(y, eb, w - 1, w > 0);
-            epilogue<RM, POL>(t, B, pl.ep, tab, k, parts, box, y, hold, sdft, bacc);
+            epilogue<RM, POL, V>(t, B, pl.ep, tab, k, parts, box, y, hold, sdft, bacc);
         }
     }
     return bad;
