@@ -1394,9 +1394,10 @@ K3 view(const LensGrid3D *g, int rb, int wb) {
     return k;
 }
 
-// x-chunks of the fused pass: the planes that carry x CPML psi get chunks of
-// their own, the rest is cut into pieces of about `target` planes.  Returns the
-// chunk count; x[c] is the first plane of chunk c, strip[c] != 0 for CPML chunks.
+// x-chunks of the fused pass: the planes that carry x CPML psi get chunks of their own,
+// every run cut into pieces of about `target` planes.  Returns the chunk count; x[c] is
+// the first plane of chunk c, strip[c] != 0 for CPML chunks.  Where a chunk ends changes
+// no cell's update: the plane before a chunk is recomputed from the old fields and psi.
 int make_chunks(const LensGrid3D *g, int target, int *x, int *strip) {
     const int nx = g->nx;
     int n = 0;
@@ -1411,16 +1412,20 @@ int make_chunks(const LensGrid3D *g, int target, int *x, int *strip) {
         strip[n] = s;
         x[++n] = b;
     };
-    if (lo > 0) add(0, lo, 1);
+    auto add_strip = [&](int a, int b) {
+        const int np = std::min((b - a + target - 1) / target, 16);
+        for (int q = 0; q < np; ++q) add(a + (int)((long)(b - a) * q / np), a + (int)((long)(b - a) * (q + 1) / np), 1);
+    };
+    if (lo > 0) add_strip(0, lo);
     const int mid = hi - lo;
     if (mid > 0) {
         int pieces = (mid + target / 2) / target;
         if (pieces < 1) pieces = 1;
-        if (pieces > MAXCH - 4) pieces = MAXCH - 4;
+        if (pieces > MAXCH - 34) pieces = MAXCH - 34;
         for (int q = 0; q < pieces; ++q)
             add(lo + (int)((long)mid * q / pieces), lo + (int)((long)mid * (q + 1) / pieces), 0);
     }
-    if (hi < nx) add(hi, nx, 1);
+    if (hi < nx) add_strip(hi, nx);
     return n;
 }
 
@@ -1436,19 +1441,46 @@ void lean_range(int count, F is_strip, int &l0, int &l1) {
         if (!is_strip(q)) l0 = l1 = 0;
 }
 
-// Work of the fused pass: all tiles, and the CPML-free interior core.  The chunk length is chosen so that the CTAs
-// fill whole waves of `slots` resident CTAs: estimated time = waves x (planes
-// per chunk + 1 warm-up plane).
+// Work of the fused pass: all tiles, and the CPML-free interior core.  The chunk length
+// is the one of the least estimated time on `slots` resident CTAs: a CTA takes (planes +
+// 2) x the plane time of its tile, by the axes whose psi it carries (the two planes: its
+// warm-up plane and start), a launch as long as its longest CTA, or its whole work over
+// the slots and a share of one lean chunk for the last CTAs' tail.  With chunks chosen for
+// whole waves of equal CTAs alone, at least 12 planes long, 64 x 48 x 40 cells took 51 us a
+// step (the CPML tiles' 12 planes one after another) and 200 x 100 x 120 took 97.
+constexpr int PLANE_COST[4] = {10, 14, 19, 23};  // tenths of a lean plane (1.6 us), by axes
 Work make_work(const LensGrid3D *g, int slots) {
     Work wk{};
     int cstrip[MAXCH];
     const int ntz = g->pitch / TK, nty = (g->ny + TJ - 1) / TJ;
+    // tiles / chunks without psi of an axis (a contiguous run, else none: every
+    // tile then carries that axis, which is always correct)
+    lean_range(ntz, [&](int t) {
+        const int k0 = t * TK;
+        return meets(k0 - 1, k0 + TK - 1, g->az.h) || meets(k0, k0 + TK - 1, g->az.e);
+    }, wk.plo[0], wk.phi[0]);
+    lean_range(nty, [&](int t) {
+        const int j0 = t * TJ;
+        return meets(j0 - 1, j0 + TJ - 1, g->ay.h) || meets(j0, j0 + TJ - 1, g->ay.e);
+    }, wk.plo[1], wk.phi[1]);
+    const long sz = ntz - (wk.phi[0] - wk.plo[0]), sy = nty - (wk.phi[1] - wk.plo[1]);  // strip tiles
+    const long tiles[3] = {(ntz - sz) * (nty - sy), sz * (nty - sy) + (ntz - sz) * sy, sz * sy};
     int target = 32;
     double best = 1e300;
-    for (int t = 12; t <= 96; t += 2) {
+    for (int t = 2; t <= 96; t += t < 12 ? 1 : 2) {
         const int nc = make_chunks(g, t, wk.x, cstrip);
-        const double waves = std::ceil((double)ntz * nty * nc / (slots > 0 ? slots : 1));
-        const double cost = waves * ((double)g->nx / nc + 1.0);
+        double total = 0.0, longest = 0.0, lean = 0.0;
+        for (int c = 0; c < nc; ++c) {
+            const double len = wk.x[c + 1] - wk.x[c] + 2.0;
+            if (cstrip[c] == 0) lean = std::max(lean, len);
+            for (int a = 0; a < 3; ++a) {
+                if (tiles[a] == 0) continue;
+                const double w = PLANE_COST[a + (cstrip[c] != 0)] * 0.1 * len;
+                total += tiles[a] * w;
+                longest = std::max(longest, w);
+            }
+        }
+        const double cost = std::max(longest, total / (slots > 0 ? slots : 1) + 0.35 * lean);
         if (cost < best - 1e-9) {
             best = cost;
             target = t;
@@ -1469,16 +1501,6 @@ Work make_work(const LensGrid3D *g, int slots) {
                j0 + TJ - 1 > g->ny - 2;
     }, y0, y1);
     lean_range(nc, [&](int c) { return cstrip[c] != 0 || wk.x[c] < 1 || wk.x[c + 1] > g->nx - 1; }, c0, c1);
-    // tiles / chunks without psi of an axis (a contiguous run, else none: every
-    // tile then carries that axis, which is always correct)
-    lean_range(ntz, [&](int t) {
-        const int k0 = t * TK;
-        return meets(k0 - 1, k0 + TK - 1, g->az.h) || meets(k0, k0 + TK - 1, g->az.e);
-    }, wk.plo[0], wk.phi[0]);
-    lean_range(nty, [&](int t) {
-        const int j0 = t * TJ;
-        return meets(j0 - 1, j0 + TJ - 1, g->ay.h) || meets(j0, j0 + TJ - 1, g->ay.e);
-    }, wk.plo[1], wk.phi[1]);
     lean_range(nc, [&](int c) {
         const int a = wk.x[c], b = wk.x[c + 1];
         return meets(a > 0 ? a - 1 : 0, b - 1, g->ax.h) || meets(a, b - 1, g->ax.e);
