@@ -144,6 +144,15 @@ int lens_te2d_step(const LensTE2D *g, const LensStepTable *tab, const LensEpi2D 
 int lens_tm2d_step(const LensTM2D *g, const LensStepTable *tab, const LensEpi2D *ep,
                    int n0, int nsteps, void *stream);
 
+/* The same steps reading the coefficients of row rowref[i] for row i (device array of nx
+ * ints, 0 <= rowref[i] < nx; NULL: every row its own): a layered grid repeats a few rows,
+ * which then come from the caches instead of memory.  Row rowref[i] must hold row i's
+ * coefficients bit for bit, in every coefficient array.                        */
+int lens_te2d_step_rows(const LensTE2D *g, const int *rowref, const LensStepTable *tab, const LensEpi2D *ep,
+                        int n0, int nsteps, void *stream);
+int lens_tm2d_step_rows(const LensTM2D *g, const int *rowref, const LensStepTable *tab, const LensEpi2D *ep,
+                        int n0, int nsteps, void *stream);
+
 /* Stitch-window drive of a 2D grid (fdtd2d_core.py:1439-1440, 1462-1463): after
  * each E update, before the PEC termination, the first nplanes x-rows of the
  * driven component (TE: Ez, TM: Ey) become

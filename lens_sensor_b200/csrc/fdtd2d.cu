@@ -15,6 +15,9 @@
 //       Ey += -Ca_ey*(...)                                               (:249-258)
 // then the Huygens source (vcsel.py:151-156) and the PEC termination
 // (boundaries.py:207-215, 260-268) in the reference order (inject, then PEC).
+#include <algorithm>
+#include <initializer_list>
+
 #include "lens_common.cuh"
 
 namespace {
@@ -30,13 +33,27 @@ __device__ __forceinline__ float src_term(const LensSource &s, const LensStepTab
     return -((tab.env[k] * sinf(tab.wt[k] + s.ph2[j])) * s.amp[j]);
 }
 
+// Compensated complex sum of v e^{-iwt} (lens_common.cuh's kahan_add with its first product
+// fused, written out so that every kernel rounds alike).
+__device__ __forceinline__ void kahan_node(float *p, size_t o, float v, float pr, float pi) {
+    float4 a = reinterpret_cast<float4 *>(p)[o];
+    float y = __fmaf_rn(v, pr, -a.z), t = __fadd_rn(a.x, y);
+    a.z = __fsub_rn(__fsub_rn(t, a.x), y);
+    a.x = t;
+    y = __fmaf_rn(v, pi, -a.w);
+    t = __fadd_rn(a.y, y);
+    a.w = __fsub_rn(__fsub_rn(t, a.y), y);
+    a.y = t;
+    reinterpret_cast<float4 *>(p)[o] = a;
+}
+
 // Epilogue on one node: detector boxes (FP64), compensated DFTs, intensity average.
 // Every lane of the warp must call it (the box sums use warp shuffles).
 __device__ __forceinline__ void epilogue_node(const LensEpi2D &ep, const LensStepTable &tab,
                                               int n, int i, int j, bool valid, size_t o,
-                                              float field, float inten, float exn) {
+                                              float field, float inten, float exn, int bx_, int by_) {
     if (ep.nbox > 0) {
-        const int bi0 = blockIdx.y * BY, bj0 = blockIdx.x * BX;
+        const int bi0 = by_ * BY, bj0 = bx_ * BX;
         for (int b = 0; b < ep.nbox; ++b) {
             const int *bx = ep.box[b];
             // block-uniform test: does this block touch box b at all?
@@ -49,14 +66,14 @@ __device__ __forceinline__ void epilogue_node(const LensEpi2D &ep, const LensSte
     const int k = n - tab.t0;
     if (n >= ep.dft_n0 && n < ep.dft_n1) {
         const float pr = tab.pe[2 * k], pi = tab.pe[2 * k + 1];
-        if (ep.dft) kahan_add(reinterpret_cast<float4 *>(ep.dft) + o, field * pr, field * pi);
-        if (ep.dft_ex) kahan_add(reinterpret_cast<float4 *>(ep.dft_ex) + o, exn * pr, exn * pi);
+        if (ep.dft) kahan_node(ep.dft, o, field, pr, pi);
+        if (ep.dft_ex) kahan_node(ep.dft_ex, o, exn, pr, pi);
     }
     if (ep.dft_prev && n >= ep.prev_n0 && n < ep.prev_n1) {
         const float pr = tab.pe[2 * k], pi = tab.pe[2 * k + 1];
-        kahan_add(reinterpret_cast<float4 *>(ep.dft_prev) + o, field * pr, field * pi);
+        kahan_node(ep.dft_prev, o, field, pr, pi);
     }
-    if (ep.iavg && n >= ep.iavg_n0) ep.iavg[o] += inten;
+    if (ep.iavg && n >= ep.iavg_n0) ep.iavg[o] = __fadd_rn(ep.iavg[o], inten);
 }
 
 // Plane DFT for the Poynting flux (flux.py:28-41): E on the plane, H averaged.
@@ -171,7 +188,7 @@ __global__ void __launch_bounds__(BX *BY)
         for (int p = 0; p < ep.nsx; ++p)
             if (i == ep.sx_plane[p]) sx_node(ep, p, P, j, ez, g.hy[o - P], g.hy[o]);
     }
-    epilogue_node(ep, tab, n, i, j, valid, o, ez, ez * ez, 0.f);
+    epilogue_node(ep, tab, n, i, j, valid, o, ez, __fmul_rn(ez, ez), 0.f, blockIdx.x, blockIdx.y);
 }
 
 // ------------------------------------------------------------------ TM
@@ -246,9 +263,10 @@ __global__ void __launch_bounds__(BX *BY)
 
 // Node averages of the new TM fields (fdtd2d_core.py:458-486) and the epilogue.
 __global__ void __launch_bounds__(BX *BY)
-    tm2d_epi(const LensTM2D g, const LensStepTable tab, const LensEpi2D ep, int n) {
-    const int j = blockIdx.x * BX + threadIdx.x;
-    const int i = blockIdx.y * BY + threadIdx.y;
+    tm2d_epi(const LensTM2D g, const LensStepTable tab, const LensEpi2D ep, int n, int bx0, int by0) {
+    const int bx = blockIdx.x + bx0, by = blockIdx.y + by0;  // blocks (bx0, by0) on of the grid
+    const int j = bx * BX + threadIdx.x;
+    const int i = by * BY + threadIdx.y;
     const bool valid = i < g.nx && j < g.ny;
     const int P = g.pitch;
     const size_t o = (size_t)i * P + j;
@@ -268,10 +286,10 @@ __global__ void __launch_bounds__(BX *BY)
             exn = a;
         } else {
             const float a = g.ex[o - P], b = g.ex[o];
-            s2 = 0.5f * (a * a + b * b);
+            s2 = 0.5f * __fmaf_rn(a, a, __fmul_rn(b, b));
             exn = 0.5f * (a + b);
         }
-        inten = field * field + s2;
+        inten = __fmaf_rn(field, field, s2);
         if (in_window(ep, n)) {  // stitch: Ey on its own grid, Ex^2 on the nodes
             if (ep.dft_raw && j < ny - 1) {
                 const int k = n - tab.t0;
@@ -289,17 +307,279 @@ __global__ void __launch_bounds__(BX *BY)
             for (int p = 0; p < ep.nsx; ++p)
                 if (i == ep.sx_plane[p]) sx_node(ep, p, P, j, g.ey[o], g.hz[o - P], g.hz[o]);
     }
-    epilogue_node(ep, tab, n, i, j, valid, o, field, inten, exn);
+    epilogue_node(ep, tab, n, i, j, valid, o, field, inten, exn, bx, by);
 }
 
-bool epi2d_active(const LensEpi2D *ep, int n) {
+// ------------------------------------------------------------------ wide passes
+// H and E passes of grids too large for the chip (grid2d_resident.cuh): a thread updates
+// WV = 4 columns of WR = 4 rows, all of its 16-byte loads issued before the arithmetic.
+// They stream: 16 B (H) and 20 B (E) a cell for TM, 20 and 16 for TE, plus the
+// coefficients, whose rows a layered grid repeats: rowref names the row to read, so a
+// repeated row comes from the caches (NULL: every row its own).  One cell a thread (the
+// kernels above, for the forms only they carry) ran 16000 x 700 TM cells at 298 us a step,
+// 1.95 TB/s: too few bytes in flight.
+// The multiply-adds are written out and round as those kernels do, and as
+// grid2d_resident.cuh.
+constexpr int WV = 4, WR = 4, WT = 8;   // columns, rows of a thread; warps of a block (along x)
+
+__device__ __forceinline__ float psi_w(const LensProfile &p, int m, float *q, float d) {
+    const float v = __fmaf_rn(__ldg(p.b + m), *q, __fmul_rn(__ldg(p.c + m), d));
+    *q = v;
+    return v;
+}
+
+__device__ __forceinline__ void ld4(float (&v)[WV], const float *p, bool on) {
+    const float4 t = on ? *reinterpret_cast<const float4 *>(p) : make_float4(0.f, 0.f, 0.f, 0.f);
+    v[0] = t.x; v[1] = t.y; v[2] = t.z; v[3] = t.w;
+}
+
+__device__ __forceinline__ void st4(float *p, const float (&v)[WV]) {
+    *reinterpret_cast<float4 *>(p) = make_float4(v[0], v[1], v[2], v[3]);
+}
+
+// First row and column of this thread; rows of the last block may lie beyond nx (no
+// return before the shuffles below: whole warps share their rows).
+__device__ __forceinline__ int wide_i0() { return (blockIdx.y * WT + threadIdx.y) * WR; }
+__device__ __forceinline__ int wide_j0() { return (blockIdx.x * BX + threadIdx.x) * WV; }
+
+// Value of the column after (up) / before (dn) a lane's four; the warp's last / first lane loads it.
+__device__ __forceinline__ float wide_up(const float (&v)[WV], const float *row, int j0, bool on) {
+    const float u = __shfl_down_sync(0xffffffffu, v[0], 1);
+    return threadIdx.x == 31 ? (on ? row[j0 + WV] : 0.f) : u;
+}
+__device__ __forceinline__ float wide_dn(const float (&v)[WV], const float *row, int j0, bool on) {
+    const float u = __shfl_up_sync(0xffffffffu, v[WV - 1], 1);
+    return threadIdx.x == 0 ? (on ? row[j0 - 1] : 0.f) : u;
+}
+
+__global__ void __launch_bounds__(32 * WT) te2d_h_wide(const LensTE2D g) {
+    const int i0 = wide_i0(), j0 = wide_j0(), nx = g.nx, ny = g.ny, P = g.pitch;
+    if (i0 >= nx) return;
+    const bool col = j0 < ny;  // the four columns lie inside the row pitch then
+    const size_t o = (size_t)i0 * P + j0;
+    float ez[WR + 1][WV], hx[WR][WV], hy[WR][WV], up[WR];
+#pragma unroll
+    for (int r = 0; r <= WR; ++r) ld4(ez[r], g.ez + o + (size_t)r * P, col && i0 + r < nx);
+#pragma unroll
+    for (int r = 0; r < WR; ++r) {
+        const bool in = col && i0 + r < nx;
+        ld4(hx[r], g.hx + o + (size_t)r * P, in);
+        ld4(hy[r], g.hy + o + (size_t)r * P, in);
+        up[r] = wide_up(ez[r], g.ez + (size_t)(i0 + r) * P, j0, in && j0 + WV < ny);
+    }
+    if (!col) return;
+    const int wy = g.ay.h.lo + g.ay.h.hi;
+#pragma unroll
+    for (int r = 0; r < WR; ++r) {
+        const int i = i0 + r;
+        if (i >= nx) break;
+        const int s = i < nx - 1 ? strip_of(i, g.ax.h.lo, g.ax.h.hi, g.ax.h.n) : -1;
+        const float kx = i < nx - 1 ? __ldg(g.ax.h.ik + i) : 0.f;
+#pragma unroll
+        for (int c = 0; c < WV; ++c) {
+            const int j = j0 + c;
+            if (j < ny - 1) {
+                const float d = (c + 1 < WV ? ez[r][c + 1 < WV ? c + 1 : 0] : up[r]) - ez[r][c];
+                const int sj = strip_of(j, g.ay.h.lo, g.ay.h.hi, g.ay.h.n);
+                const float p = sj >= 0 ? psi_w(g.ay.h, j, g.psi_hxy + (size_t)i * wy + sj, d) : 0.f;
+                hx[r][c] = __fmaf_rn(-g.ch, __fmaf_rn(d, __ldg(g.ay.h.ik + j), p), hx[r][c]);
+            }
+            if (i < nx - 1 && j < ny) {
+                const float d = ez[r + 1][c] - ez[r][c];
+                const float p = s >= 0 ? psi_w(g.ax.h, i, g.psi_hyx + (size_t)s * P + j, d) : 0.f;
+                hy[r][c] = __fmaf_rn(g.ch, __fmaf_rn(d, kx, p), hy[r][c]);
+            }
+        }
+        st4(g.hx + o + (size_t)r * P, hx[r]);
+        if (i < nx - 1) st4(g.hy + o + (size_t)r * P, hy[r]);
+    }
+}
+
+__global__ void __launch_bounds__(32 * WT) te2d_e_wide(const LensTE2D g, const int *rowref, const LensStepTable tab, int n) {
+    const int i0 = wide_i0(), j0 = wide_j0(), nx = g.nx, ny = g.ny, P = g.pitch;
+    if (i0 >= nx) return;
+    const bool col = j0 < ny;
+    const size_t o = (size_t)i0 * P + j0;
+    float hy[WR + 1][WV], hx[WR][WV], ez[WR][WV], c0[WR][WV], c1[WR][WV], dn[WR];
+#pragma unroll
+    for (int r = 0; r <= WR; ++r)  // hy[r] = Hy(i0 + r - 1)
+        ld4(hy[r], g.hy + o + (size_t)r * P - P, col && i0 + r >= 1 && i0 + r - 1 < nx);
+#pragma unroll
+    for (int r = 0; r < WR; ++r) {
+        const int i = i0 + r;
+        const bool in = col && i < nx;
+        const size_t oc = (size_t)(in && rowref ? __ldg(rowref + i) : i) * P + j0;
+        ld4(hx[r], g.hx + o + (size_t)r * P, in);
+        ld4(ez[r], g.ez + o + (size_t)r * P, in);
+        ld4(c0[r], g.ce_e + oc, in);
+        ld4(c1[r], g.ce_h + oc, in);
+        dn[r] = wide_dn(hx[r], g.hx + (size_t)i * P, j0, in && j0 > 0);
+    }
+    if (!col) return;
+    const int wy = g.ay.e.lo + g.ay.e.hi;
+#pragma unroll
+    for (int r = 0; r < WR; ++r) {
+        const int i = i0 + r;
+        if (i >= nx) break;
+        const bool xin = i > 0 && i < nx - 1, xsrc = g.src.ix >= 0 && (i == g.src.ix || i == g.src.ix + 1);
+        const int s = xin ? strip_of(i, g.ax.e.lo, g.ax.e.hi, g.ax.e.n) : -1;
+        const float kx = __ldg(g.ax.e.ik + i);
+#pragma unroll
+        for (int c = 0; c < WV; ++c) {
+            const int j = j0 + c;
+            if (j >= ny) continue;
+            float v = ez[r][c];
+            if (xin && j > 0 && j < ny - 1) {
+                const float dhy = hy[r + 1][c] - hy[r][c], dhx = hx[r][c] - (c > 0 ? hx[r][c > 0 ? c - 1 : 0] : dn[r]);
+                const int sj = strip_of(j, g.ay.e.lo, g.ay.e.hi, g.ay.e.n);
+                const float qx = s >= 0 ? psi_w(g.ax.e, i, g.psi_ezx + (size_t)s * P + j, dhy) : 0.f;
+                const float qy = sj >= 0 ? psi_w(g.ay.e, j, g.psi_ezy + (size_t)i * wy + sj, dhx) : 0.f;
+                const float t = __fsub_rn(__fmaf_rn(-dhx, __ldg(g.ay.e.ik + j), __fmaf_rn(dhy, kx, qx)), qy);
+                v = __fmaf_rn(c0[r][c], v, __fmul_rn(c1[r][c], t));
+            }
+            if (xsrc && j < g.src.nj) v = __fadd_rn(v, src_term(g.src, tab, n, i, j));
+            if ((g.pec[0] && i == 0) || (g.pec[1] && i == nx - 1) || (g.pec[2] && j == 0) || (g.pec[3] && j == ny - 1)) v = 0.f;
+            ez[r][c] = v;
+        }
+        st4(g.ez + o + (size_t)r * P, ez[r]);
+    }
+}
+
+__global__ void __launch_bounds__(32 * WT) tm2d_h_wide(const LensTM2D g) {
+    const int i0 = wide_i0(), j0 = wide_j0(), nx = g.nx, ny = g.ny, P = g.pitch;
+    if (i0 >= nx - 1) return;
+    const bool col = j0 < ny;
+    const size_t o = (size_t)i0 * P + j0;
+    float ey[WR + 1][WV], ex[WR][WV], hz[WR][WV], up[WR];
+#pragma unroll
+    for (int r = 0; r <= WR; ++r) ld4(ey[r], g.ey + o + (size_t)r * P, col && i0 + r < nx);
+#pragma unroll
+    for (int r = 0; r < WR; ++r) {
+        const bool in = col && i0 + r < nx - 1;
+        ld4(ex[r], g.ex + o + (size_t)r * P, in);
+        ld4(hz[r], g.hz + o + (size_t)r * P, in);
+        up[r] = wide_up(ex[r], g.ex + (size_t)(i0 + r) * P, j0, in && j0 + WV < ny);
+    }
+    if (!col) return;
+    const int wy = g.ay.h.lo + g.ay.h.hi;
+#pragma unroll
+    for (int r = 0; r < WR; ++r) {
+        const int i = i0 + r;
+        if (i >= nx - 1) break;
+        const int s = strip_of(i, g.ax.h.lo, g.ax.h.hi, g.ax.h.n);
+        const float kx = __ldg(g.ax.h.ik + i);
+#pragma unroll
+        for (int c = 0; c < WV; ++c) {
+            const int j = j0 + c;
+            if (j >= ny - 1) continue;
+            const float dyx = ey[r + 1][c] - ey[r][c], dxy = (c + 1 < WV ? ex[r][c + 1 < WV ? c + 1 : 0] : up[r]) - ex[r][c];
+            const int sj = strip_of(j, g.ay.h.lo, g.ay.h.hi, g.ay.h.n);
+            const float px = s >= 0 ? psi_w(g.ax.h, i, g.psi_hzx + (size_t)s * P + j, dyx) : 0.f;
+            const float py = sj >= 0 ? psi_w(g.ay.h, j, g.psi_hzy + (size_t)i * wy + sj, dxy) : 0.f;
+            const float t = __fsub_rn(__fmaf_rn(dyx, kx, px), __fmaf_rn(dxy, __ldg(g.ay.h.ik + j), py));
+            hz[r][c] = __fmaf_rn(-g.ch, t, hz[r][c]);
+        }
+        st4(g.hz + o + (size_t)r * P, hz[r]);
+    }
+}
+
+__global__ void __launch_bounds__(32 * WT) tm2d_e_wide(const LensTM2D g, const int *rowref, const LensStepTable tab, int n) {
+    const int i0 = wide_i0(), j0 = wide_j0(), nx = g.nx, ny = g.ny, P = g.pitch;
+    if (i0 >= nx) return;
+    const bool col = j0 < ny, lossy = g.da_x != nullptr;
+    const size_t o = (size_t)i0 * P + j0;
+    float hz[WR + 1][WV], ex[WR][WV], ey[WR][WV], dn[WR];
+#pragma unroll
+    for (int r = 0; r <= WR; ++r)  // hz[r] = Hz(i0 + r - 1)
+        ld4(hz[r], g.hz + o + (size_t)r * P - P, col && i0 + r >= 1 && i0 + r - 1 < nx - 1);
+#pragma unroll
+    for (int r = 0; r < WR; ++r) {
+        const int i = i0 + r;
+        const bool inx = col && i < nx - 1, iny = col && i < nx;
+        ld4(ex[r], g.ex + o + (size_t)r * P, inx);
+        ld4(ey[r], g.ey + o + (size_t)r * P, iny);
+        dn[r] = wide_dn(hz[r + 1], g.hz + (size_t)i * P, j0, inx && j0 > 0);
+    }
+    if (!col) return;
+    const int wy = g.ay.e.lo + g.ay.e.hi;
+#pragma unroll
+    for (int r = 0; r < WR; ++r) {
+        const int i = i0 + r;
+        if (i >= nx) break;
+        const size_t oc = (size_t)(rowref ? __ldg(rowref + i) : i) * P + j0;
+        const size_t ox = i < nx - 1 ? oc : 0;  // the last row has no Ex (and no coefficients of it)
+        float ca[WV], cb[WV], da[WV], db[WV];
+        ld4(ca, g.ca_x + ox, true);
+        ld4(cb, g.ca_y + oc, true);
+        if (lossy) {
+            ld4(da, g.da_x + ox, true);
+            ld4(db, g.da_y + oc, true);
+        }
+        const bool xin = i > 0 && i < nx - 1, xsrc = g.src.ix >= 0 && (i == g.src.ix || i == g.src.ix + 1);
+        const int s = xin ? strip_of(i, g.ax.e.lo, g.ax.e.hi, g.ax.e.n) : -1;
+        const float kx = __ldg(g.ax.e.ik + i);
+#pragma unroll
+        for (int c = 0; c < WV; ++c) {
+            const int j = j0 + c;
+            if (i < nx - 1 && j < ny) {  // Ex at (i+1/2, j)
+                float e = ex[r][c];
+                if (lossy) e = __fmul_rn(e, da[c]);
+                if (j > 0 && j < ny - 1) {
+                    const float d = hz[r + 1][c] - (c > 0 ? hz[r + 1][c > 0 ? c - 1 : 0] : dn[r]);
+                    const int sj = strip_of(j, g.ay.e.lo, g.ay.e.hi, g.ay.e.n);
+                    const float p = sj >= 0 ? psi_w(g.ay.e, j, g.psi_exy + (size_t)i * wy + sj, d) : 0.f;
+                    e = __fmaf_rn(ca[c], __fmaf_rn(d, __ldg(g.ay.e.ik + j), p), e);
+                }
+                if ((g.pec[2] && j == 0) || (g.pec[3] && j == ny - 1)) e = 0.f;
+                ex[r][c] = e;
+            }
+            if (j < ny - 1) {  // Ey at (i, j+1/2)
+                float e = ey[r][c];
+                if (lossy) e = __fmul_rn(e, db[c]);
+                if (xin) {
+                    const float d = hz[r + 1][c] - hz[r][c];
+                    const float p = s >= 0 ? psi_w(g.ax.e, i, g.psi_eyx + (size_t)s * P + j, d) : 0.f;
+                    e = __fmaf_rn(-cb[c], __fmaf_rn(d, kx, p), e);
+                }
+                if (xsrc && j < g.src.nj) e = __fadd_rn(e, src_term(g.src, tab, n, i, j));
+                if ((g.pec[0] && i == 0) || (g.pec[1] && i == nx - 1)) e = 0.f;
+                ey[r][c] = e;
+            }
+        }
+        if (i < nx - 1) st4(g.ex + o + (size_t)r * P, ex[r]);
+        st4(g.ey + o + (size_t)r * P, ey[r]);
+    }
+}
+
+// Epilogue of the new Ez after a wide E pass, blocks (bx0, by0) on of the grid.
+__global__ void __launch_bounds__(BX *BY)
+    te2d_epi(const LensTE2D g, const LensStepTable tab, const LensEpi2D ep, int n, int bx0, int by0) {
+    const int bx = blockIdx.x + bx0, by = blockIdx.y + by0;
+    const int j = bx * BX + threadIdx.x, i = by * BY + threadIdx.y;
+    const bool valid = i < g.nx && j < g.ny;
+    const int P = g.pitch;
+    const size_t o = (size_t)i * P + j;
+    float ez = 0.f;
+    if (valid) {
+        ez = g.ez[o];
+        if (ep.nplane > 0 && in_window(ep, n))
+            for (int p = 0; p < ep.nplane; ++p)
+                if (i == ep.plane[p]) plane_node(ep, tab, n, p, P, j, ez, 0.5f * (g.hy[o - P] + g.hy[o]));
+    }
+    epilogue_node(ep, tab, n, i, j, valid, o, ez, __fmul_rn(ez, ez), 0.f, bx, by);
+}
+
+// Does the epilogue do more at step n than sum its boxes?
+bool epi2d_beyond_boxes(const LensEpi2D *ep, int n) {
     if (!ep) return false;
-    if (ep->nbox > 0 || ep->nsx > 0) return true;
+    if (ep->nsx > 0) return true;
     if ((ep->dft || ep->dft_ex || ep->dft_raw || ep->ex2 || ep->nplane > 0) && n >= ep->dft_n0 && n < ep->dft_n1)
         return true;
     if (ep->dft_prev && n >= ep->prev_n0 && n < ep->prev_n1) return true;
     return ep->iavg && n >= ep->iavg_n0;
 }
+
+bool epi2d_active(const LensEpi2D *ep, int n) { return epi2d_beyond_boxes(ep, n) || (ep && ep->nbox > 0); }
 
 bool epi2d_ok(const LensEpi2D *ep, const LensStepTable *t, int nx) {
     if (!ep) return true;
@@ -348,8 +628,37 @@ bool drive2d_ok(const LensDrive2D *d, const LensStepTable *tab, int nx) {
                                      (reinterpret_cast<uintptr_t>(d->hand) & 7) == 0 && tab);
 }
 
+// The wide passes carry every plain step whose arrays start on 16-byte boundaries; the
+// stitch drive, the stitch sums and the pulse planes stay with one cell a thread.
+bool wide_ok(const LensEpi2D &e, const LensDrive2D *dr, std::initializer_list<const void *> arrays) {
+    if (dr || e.nsx > 0 || e.dft_raw || e.ex2) return false;
+    for (const void *p : arrays)
+        if (reinterpret_cast<uintptr_t>(p) & 15) return false;
+    return true;
+}
+
+// Epilogue of a wide step: every block of the grid, or on steps that only sum boxes the
+// blocks of each box (run once with the other boxes' extents empty).
+template <class F>
+void wide_epilogue(const LensEpi2D &e, int n, int nx, int ny, F launch) {
+    if (epi2d_beyond_boxes(&e, n)) {
+        launch(e, 0, 0, (ny + BX - 1) / BX, (nx + BY - 1) / BY);
+        return;
+    }
+    for (int b = 0; b < e.nbox; ++b) {
+        const int i0 = std::max(0, e.box[b][0]), i1 = std::min(nx, e.box[b][1]), j0 = std::max(0, e.box[b][2]),
+                  j1 = std::min(ny, e.box[b][3]);
+        if (i1 <= i0 || j1 <= j0) continue;
+        LensEpi2D one = e;
+        one.nbox = 1;
+        for (int q = 0; q < 4; ++q) one.box[0][q] = e.box[b][q];
+        one.box_acc = e.box_acc + b;
+        launch(one, j0 / BX, i0 / BY, (j1 + BX - 1) / BX - j0 / BX, (i1 + BY - 1) / BY - i0 / BY);
+    }
+}
+
 int te2d_run(const LensTE2D *g, const LensStepTable *tab, const LensEpi2D *ep, const LensDrive2D *dr, int n0,
-             int nsteps, void *stream) {
+             int nsteps, void *stream, const int *rowref = nullptr) {
     if (!grid2d_ok(g) || !psi2d_ok(g) || !g->ez || !g->hx || !g->hy || !g->ce_e || !g->ce_h || nsteps < 0 ||
         !lens_table_ok(tab, n0, nsteps) || !epi2d_ok(ep, tab, g->nx) || !drive2d_ok(dr, tab, g->nx))
         return LENS_ERR_ARG;
@@ -357,6 +666,17 @@ int te2d_run(const LensTE2D *g, const LensStepTable *tab, const LensEpi2D *ep, c
     const LensDrive2D d = dr ? *dr : LensDrive2D{};
     cudaStream_t s = static_cast<cudaStream_t>(stream);
     const dim3 blk(BX, BY), grd((g->ny + BX - 1) / BX, (g->nx + BY - 1) / BY);
+    if (wide_ok(e, dr, {g->ez, g->hx, g->hy, g->ce_e, g->ce_h})) {
+        const dim3 wb(BX, WT), wg((g->ny + BX * WV - 1) / (BX * WV), (g->nx + WT * WR - 1) / (WT * WR));
+        for (int n = n0; n < n0 + nsteps; ++n) {
+            te2d_h_wide<<<wg, wb, 0, s>>>(*g);
+            te2d_e_wide<<<wg, wb, 0, s>>>(*g, rowref, *tab, n);
+            wide_epilogue(e, n, g->nx, g->ny, [&](const LensEpi2D &v, int bx, int by, int wx, int wy) {
+                te2d_epi<<<dim3(wx, wy), blk, 0, s>>>(*g, *tab, v, n, bx, by);
+            });
+        }
+        return lens_cuda_status();
+    }
     for (int n = n0; n < n0 + nsteps; ++n) {
         te2d_h<<<grd, blk, 0, s>>>(*g);
         te2d_e<<<grd, blk, 0, s>>>(*g, *tab, e, n, d);
@@ -365,7 +685,7 @@ int te2d_run(const LensTE2D *g, const LensStepTable *tab, const LensEpi2D *ep, c
 }
 
 int tm2d_run(const LensTM2D *g, const LensStepTable *tab, const LensEpi2D *ep, const LensDrive2D *dr, int n0,
-             int nsteps, void *stream) {
+             int nsteps, void *stream, const int *rowref = nullptr) {
     if (!grid2d_ok(g) || !psi2d_ok(g) || !g->ex || !g->ey || !g->hz || !g->ca_x || !g->ca_y ||
         (!g->da_x) != (!g->da_y) || nsteps < 0 || !lens_table_ok(tab, n0, nsteps) ||
         !epi2d_ok(ep, tab, g->nx) || !drive2d_ok(dr, tab, g->nx))
@@ -374,10 +694,21 @@ int tm2d_run(const LensTM2D *g, const LensStepTable *tab, const LensEpi2D *ep, c
     const LensDrive2D d = dr ? *dr : LensDrive2D{};
     cudaStream_t s = static_cast<cudaStream_t>(stream);
     const dim3 blk(BX, BY), grd((g->ny + BX - 1) / BX, (g->nx + BY - 1) / BY);
+    if (wide_ok(e, dr, {g->ex, g->ey, g->hz, g->ca_x, g->ca_y, g->da_x, g->da_y})) {
+        const dim3 wb(BX, WT), wg((g->ny + BX * WV - 1) / (BX * WV), (g->nx + WT * WR - 1) / (WT * WR));
+        for (int n = n0; n < n0 + nsteps; ++n) {
+            tm2d_h_wide<<<wg, wb, 0, s>>>(*g);
+            tm2d_e_wide<<<wg, wb, 0, s>>>(*g, rowref, *tab, n);
+            wide_epilogue(e, n, g->nx, g->ny, [&](const LensEpi2D &v, int bx, int by, int wx, int wy) {
+                tm2d_epi<<<dim3(wx, wy), blk, 0, s>>>(*g, *tab, v, n, bx, by);
+            });
+        }
+        return lens_cuda_status();
+    }
     for (int n = n0; n < n0 + nsteps; ++n) {
         tm2d_h<<<grd, blk, 0, s>>>(*g);
         tm2d_e<<<grd, blk, 0, s>>>(*g, *tab, n, d);
-        if (epi2d_active(&e, n)) tm2d_epi<<<grd, blk, 0, s>>>(*g, *tab, e, n);
+        if (epi2d_active(&e, n)) tm2d_epi<<<grd, blk, 0, s>>>(*g, *tab, e, n, 0, 0);
     }
     return lens_cuda_status();
 }
@@ -392,6 +723,16 @@ extern "C" int lens_te2d_step(const LensTE2D *g, const LensStepTable *tab, const
 extern "C" int lens_tm2d_step(const LensTM2D *g, const LensStepTable *tab, const LensEpi2D *ep,
                               int n0, int nsteps, void *stream) {
     return tm2d_run(g, tab, ep, nullptr, n0, nsteps, stream);
+}
+
+extern "C" int lens_te2d_step_rows(const LensTE2D *g, const int *rowref, const LensStepTable *tab, const LensEpi2D *ep,
+                                   int n0, int nsteps, void *stream) {
+    return te2d_run(g, tab, ep, nullptr, n0, nsteps, stream, rowref);
+}
+
+extern "C" int lens_tm2d_step_rows(const LensTM2D *g, const int *rowref, const LensStepTable *tab, const LensEpi2D *ep,
+                                   int n0, int nsteps, void *stream) {
+    return tm2d_run(g, tab, ep, nullptr, n0, nsteps, stream, rowref);
 }
 
 extern "C" int lens_te2d_step_driven(const LensTE2D *g, const LensStepTable *tab, const LensEpi2D *ep,

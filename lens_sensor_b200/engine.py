@@ -62,6 +62,19 @@ def strip_widths(c):
     return lo, hi
 
 
+def repeated_rows(arrays):
+    """For every row of the (nx, pitch) arrays the first row of the run of equal rows it
+    lies in (equal bit for bit in all of them), int32 on the arrays' device."""
+    nx = arrays[0].shape[0]
+    new = torch.zeros(nx, dtype=torch.bool, device=arrays[0].device)
+    new[0] = True
+    for a in arrays:
+        b = a.view(torch.int32)
+        new[1:] |= (b[1:] != b[:-1]).any(dim=1)
+    idx = torch.arange(nx, dtype=torch.int32, device=new.device)
+    return torch.cummax(torch.where(new, idx, torch.zeros_like(idx)), dim=0).values.to(torch.int32)
+
+
 # Steps from which Grid2D.step takes the resident launch: a launch of few steps pays for
 # the state's way in and out (see the launch in csrc/grid2d_resident.cuh).
 RS_MIN_STEPS = 4
@@ -189,6 +202,9 @@ class Grid2D:
             ctypes.byref(self.s))
         self.rs_scratch = torch.empty(need, dtype=torch.uint8, device=dev) if need else None
         self.rs_err = torch.zeros(1, dtype=torch.int32, device=dev) if need else None
+        # coefficient rows that repeat, read once by the step by step passes of a grid beyond the chip
+        self.rowref = None if need else repeated_rows(
+            [self.ce_e, self.ce_h] if self.pol == 's' else [self.ca_x, self.ca_y] + ([self.da_x, self.da_y] if da else []))
 
     # reference-shaped views of the resident fields
     def view(self, name):
@@ -222,8 +238,9 @@ class Grid2D:
             if st != N.ERR_SIZE:      # else: a call that only the steps below carry
                 return N.check(st)
         if drive is None:
-            fn = self.lib.lens_te2d_step if self.pol == 's' else self.lib.lens_tm2d_step
-            N.check(fn(ctypes.byref(self.s), ctypes.byref(table.s), e, int(n0), int(nsteps), _stream_ptr(stream)))
+            fn = self.lib.lens_te2d_step_rows if self.pol == 's' else self.lib.lens_tm2d_step_rows
+            N.check(fn(ctypes.byref(self.s), _ptr(self.rowref), ctypes.byref(table.s), e, int(n0), int(nsteps),
+                       _stream_ptr(stream)))
         else:
             fn = self.lib.lens_te2d_step_driven if self.pol == 's' else self.lib.lens_tm2d_step_driven
             N.check(fn(ctypes.byref(self.s), ctypes.byref(table.s), e, ctypes.byref(drive.s), int(n0),

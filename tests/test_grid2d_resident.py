@@ -169,3 +169,46 @@ def test_watchdog_ends_the_launch():
     torch.cuda.synchronize()
     a.check()
     assert bool(torch.isfinite(a.ez).all())
+
+
+WIDE = [('s', 60, 33, False, {}), ('p', 61, 65, True, {}), ('p', 133, 128, False, {}), ('s', 301, 257, False, {}),
+        ('p', 300, 700, True, {}), ('s', 97, 131, False, dict(full_x=True)), ('p', 90, 70, True, dict(source=False)),
+        ('s', 64, 100, False, dict(pec=(0, 1, 0, 1))), ('p', 65, 100, True, dict(pec=(1, 0, 1, 0)))]
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize('rows', [False, True])
+@pytest.mark.parametrize('case', WIDE, ids=lambda c: f'{c[0]}-{c[1]}x{c[2]}')
+def test_wide_passes_keep_the_bits(case, rows, monkeypatch):
+    """The four-columns-a-thread passes against the one-cell-a-thread kernels (which a
+    driven step of no rows runs), coefficient rows read once or each its own."""
+    import torch
+    from lens_sensor_b200 import engine as E
+    pol, nx, ny, lossy, kw = case
+    steps = 12
+    a, b = (_grid(pol, nx, ny, lossy, 9, **kw) for _ in range(2))
+    monkeypatch.setattr(E, 'RS_MIN_STEPS', 1 << 30)
+    if rows:
+        co = [a.ce_e, a.ce_h] if pol == 's' else [a.ca_x, a.ca_y] + ([a.da_x, a.da_y] if lossy else [])
+        a.rowref = E.repeated_rows(co)
+        ref = a.rowref.cpu().numpy()
+        assert (ref <= np.arange(nx)).all() and len(set(ref.tolist())) < nx
+        for c in co:
+            assert torch.equal(c[a.rowref.long()], c)
+    tab = E.StepTable(7, steps, a.dt, 2.2e15, 2.2e15, E.cw_envelope(3.5e14))
+    ea, eb = _epi(a, steps, True), _epi(b, steps, True)
+    a.step(tab, 7, steps, ea)
+    none = N.Drive2D()
+    fn = b.lib.lens_te2d_step_driven if pol == 's' else b.lib.lens_tm2d_step_driven
+    assert fn(ctypes.byref(b.s), ctypes.byref(tab.s), ctypes.byref(eb.s), ctypes.byref(none), 7, steps, None) == 0
+    torch.cuda.synchronize()
+    for q in FIELDS[pol]:
+        assert torch.equal(getattr(a, q), getattr(b, q)), q
+    for q in b.psi:
+        assert torch.equal(a.psi[q], b.psi[q]), q
+    for q in SUMS:
+        if getattr(eb, q) is not None:
+            assert torch.equal(getattr(ea, q), getattr(eb, q)), q
+    for q in ('box_acc', 'plane_acc'):
+        x, y = getattr(ea, q), getattr(eb, q)
+        assert float((x - y).abs().max()) <= 1e-12 * max(float(y.abs().max()), 1e-300), q
