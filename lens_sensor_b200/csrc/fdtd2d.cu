@@ -51,9 +51,9 @@ __device__ __forceinline__ void kahan_node(float *p, size_t o, float v, float pr
 // Every lane of the warp must call it (the box sums use warp shuffles).
 __device__ __forceinline__ void epilogue_node(const LensEpi2D &ep, const LensStepTable &tab,
                                               int n, int i, int j, bool valid, size_t o,
-                                              float field, float inten, float exn, int bx_, int by_) {
+                                              float field, float inten, float exn) {
     if (ep.nbox > 0) {
-        const int bi0 = by_ * BY, bj0 = bx_ * BX;
+        const int bi0 = blockIdx.y * BY, bj0 = blockIdx.x * BX;
         for (int b = 0; b < ep.nbox; ++b) {
             const int *bx = ep.box[b];
             // block-uniform test: does this block touch box b at all?
@@ -188,7 +188,7 @@ __global__ void __launch_bounds__(BX *BY)
         for (int p = 0; p < ep.nsx; ++p)
             if (i == ep.sx_plane[p]) sx_node(ep, p, P, j, ez, g.hy[o - P], g.hy[o]);
     }
-    epilogue_node(ep, tab, n, i, j, valid, o, ez, __fmul_rn(ez, ez), 0.f, blockIdx.x, blockIdx.y);
+    epilogue_node(ep, tab, n, i, j, valid, o, ez, __fmul_rn(ez, ez), 0.f);
 }
 
 // ------------------------------------------------------------------ TM
@@ -263,10 +263,9 @@ __global__ void __launch_bounds__(BX *BY)
 
 // Node averages of the new TM fields (fdtd2d_core.py:458-486) and the epilogue.
 __global__ void __launch_bounds__(BX *BY)
-    tm2d_epi(const LensTM2D g, const LensStepTable tab, const LensEpi2D ep, int n, int bx0, int by0) {
-    const int bx = blockIdx.x + bx0, by = blockIdx.y + by0;  // blocks (bx0, by0) on of the grid
-    const int j = bx * BX + threadIdx.x;
-    const int i = by * BY + threadIdx.y;
+    tm2d_epi(const LensTM2D g, const LensStepTable tab, const LensEpi2D ep, int n) {
+    const int j = blockIdx.x * BX + threadIdx.x;
+    const int i = blockIdx.y * BY + threadIdx.y;
     const bool valid = i < g.nx && j < g.ny;
     const int P = g.pitch;
     const size_t o = (size_t)i * P + j;
@@ -307,20 +306,24 @@ __global__ void __launch_bounds__(BX *BY)
             for (int p = 0; p < ep.nsx; ++p)
                 if (i == ep.sx_plane[p]) sx_node(ep, p, P, j, g.ey[o], g.hz[o - P], g.hz[o]);
     }
-    epilogue_node(ep, tab, n, i, j, valid, o, field, inten, exn, bx, by);
+    epilogue_node(ep, tab, n, i, j, valid, o, field, inten, exn);
 }
 
 // ------------------------------------------------------------------ wide passes
 // H and E passes of grids too large for the chip (grid2d_resident.cuh): a thread updates
-// WV = 4 columns of WR = 4 rows, all of its 16-byte loads issued before the arithmetic.
+// WV = 4 columns of WR = 2 rows, all of its 16-byte loads issued before the arithmetic.
 // They stream: 16 B (H) and 20 B (E) a cell for TM, 20 and 16 for TE, plus the
 // coefficients, whose rows a layered grid repeats: rowref names the row to read, so a
-// repeated row comes from the caches (NULL: every row its own).  One cell a thread (the
-// kernels above, for the forms only they carry) ran 16000 x 700 TM cells at 298 us a step,
-// 1.95 TB/s: too few bytes in flight.
+// repeated row comes from the caches (NULL: every row its own).  Memory latency bounds
+// them: 16000 x 700 cells with boxes, us a step TM / TE: 298 / 290 at one cell a thread (the
+// kernels above, kept for the forms only they carry), 106 / 95 here with 32 warps an SM, 110 /
+// 98 in blocks of 8 warps, 139 / 122 without the register cap, 137 / 111 with 3 rows, 125 / 112
+// with one row and 48 warps.  Warps clear of strips, faces and source rows run without tests
+// (without that form: 178 / 165).
 // The multiply-adds are written out and round as those kernels do, and as
 // grid2d_resident.cuh.
-constexpr int WV = 4, WR = 4, WT = 8;   // columns, rows of a thread; warps of a block (along x)
+constexpr int WV = 4, WR = 2, WT = 4;   // columns, rows of a thread; warps of a block (along x)
+constexpr int WB = 8;                   // blocks of an SM: 64 registers
 
 __device__ __forceinline__ float psi_w(const LensProfile &p, int m, float *q, float d) {
     const float v = __fmaf_rn(__ldg(p.b + m), *q, __fmul_rn(__ldg(p.c + m), d));
@@ -352,7 +355,20 @@ __device__ __forceinline__ float wide_dn(const float (&v)[WV], const float *row,
     return threadIdx.x == 0 ? (on ? row[j0 - 1] : 0.f) : u;
 }
 
-__global__ void __launch_bounds__(32 * WT) te2d_h_wide(const LensTE2D g) {
+// Rows i0 .. i0+WR-1 and columns j0 .. j0+WV-1 clear of a profile pair's strips, of the faces
+// (lo: the first row and column that update) and of the source rows.
+__device__ __forceinline__ bool wide_clear(const LensProfile &x, const LensProfile &y, int i0, int j0, int nx, int ny,
+                                           int lo, int six) {
+    return i0 >= max(x.lo, lo) && i0 + WR <= min(x.n - x.hi, nx - 1) && j0 >= max(y.lo, lo) &&
+           j0 + WV <= min(y.n - y.hi, ny - 1) && (six < 0 || six + 1 < i0 || six >= i0 + WR);
+}
+
+__device__ __forceinline__ void ik4(float (&v)[WV], const float *p) {  // profile values of four columns
+#pragma unroll
+    for (int c = 0; c < WV; ++c) v[c] = __ldg(p + c);
+}
+
+__global__ void __launch_bounds__(32 * WT, WB) te2d_h_wide(const LensTE2D g) {
     const int i0 = wide_i0(), j0 = wide_j0(), nx = g.nx, ny = g.ny, P = g.pitch;
     if (i0 >= nx) return;
     const bool col = j0 < ny;  // the four columns lie inside the row pitch then
@@ -366,6 +382,23 @@ __global__ void __launch_bounds__(32 * WT) te2d_h_wide(const LensTE2D g) {
         ld4(hx[r], g.hx + o + (size_t)r * P, in);
         ld4(hy[r], g.hy + o + (size_t)r * P, in);
         up[r] = wide_up(ez[r], g.ez + (size_t)(i0 + r) * P, j0, in && j0 + WV < ny);
+    }
+    if (__all_sync(0xffffffffu, wide_clear(g.ax.h, g.ay.h, i0, j0, nx, ny, 0, -1))) {  // no psi, every cell updates
+        float ky[WV];
+        ik4(ky, g.ay.h.ik + j0);
+#pragma unroll
+        for (int r = 0; r < WR; ++r) {
+            const float kx = __ldg(g.ax.h.ik + i0 + r);
+#pragma unroll
+            for (int c = 0; c < WV; ++c) {
+                const float d = (c + 1 < WV ? ez[r][c + 1 < WV ? c + 1 : 0] : up[r]) - ez[r][c];
+                hx[r][c] = __fmaf_rn(-g.ch, __fmul_rn(d, ky[c]), hx[r][c]);
+                hy[r][c] = __fmaf_rn(g.ch, __fmul_rn(ez[r + 1][c] - ez[r][c], kx), hy[r][c]);
+            }
+            st4(g.hx + o + (size_t)r * P, hx[r]);
+            st4(g.hy + o + (size_t)r * P, hy[r]);
+        }
+        return;
     }
     if (!col) return;
     const int wy = g.ay.h.lo + g.ay.h.hi;
@@ -395,7 +428,7 @@ __global__ void __launch_bounds__(32 * WT) te2d_h_wide(const LensTE2D g) {
     }
 }
 
-__global__ void __launch_bounds__(32 * WT) te2d_e_wide(const LensTE2D g, const int *rowref, const LensStepTable tab, int n) {
+__global__ void __launch_bounds__(32 * WT, WB) te2d_e_wide(const LensTE2D g, const int *rowref, const LensStepTable tab, int n) {
     const int i0 = wide_i0(), j0 = wide_j0(), nx = g.nx, ny = g.ny, P = g.pitch;
     if (i0 >= nx) return;
     const bool col = j0 < ny;
@@ -414,6 +447,22 @@ __global__ void __launch_bounds__(32 * WT) te2d_e_wide(const LensTE2D g, const i
         ld4(c0[r], g.ce_e + oc, in);
         ld4(c1[r], g.ce_h + oc, in);
         dn[r] = wide_dn(hx[r], g.hx + (size_t)i * P, j0, in && j0 > 0);
+    }
+    if (__all_sync(0xffffffffu, wide_clear(g.ax.e, g.ay.e, i0, j0, nx, ny, 1, g.src.ix))) {
+        float ky[WV];
+        ik4(ky, g.ay.e.ik + j0);
+#pragma unroll
+        for (int r = 0; r < WR; ++r) {
+            const float kx = __ldg(g.ax.e.ik + i0 + r);
+#pragma unroll
+            for (int c = 0; c < WV; ++c) {
+                const float dhy = hy[r + 1][c] - hy[r][c], dhx = hx[r][c] - (c > 0 ? hx[r][c > 0 ? c - 1 : 0] : dn[r]);
+                const float t = __fmaf_rn(-dhx, ky[c], __fmul_rn(dhy, kx));
+                ez[r][c] = __fmaf_rn(c0[r][c], ez[r][c], __fmul_rn(c1[r][c], t));
+            }
+            st4(g.ez + o + (size_t)r * P, ez[r]);
+        }
+        return;
     }
     if (!col) return;
     const int wy = g.ay.e.lo + g.ay.e.hi;
@@ -445,7 +494,7 @@ __global__ void __launch_bounds__(32 * WT) te2d_e_wide(const LensTE2D g, const i
     }
 }
 
-__global__ void __launch_bounds__(32 * WT) tm2d_h_wide(const LensTM2D g) {
+__global__ void __launch_bounds__(32 * WT, WB) tm2d_h_wide(const LensTM2D g) {
     const int i0 = wide_i0(), j0 = wide_j0(), nx = g.nx, ny = g.ny, P = g.pitch;
     if (i0 >= nx - 1) return;
     const bool col = j0 < ny;
@@ -459,6 +508,22 @@ __global__ void __launch_bounds__(32 * WT) tm2d_h_wide(const LensTM2D g) {
         ld4(ex[r], g.ex + o + (size_t)r * P, in);
         ld4(hz[r], g.hz + o + (size_t)r * P, in);
         up[r] = wide_up(ex[r], g.ex + (size_t)(i0 + r) * P, j0, in && j0 + WV < ny);
+    }
+    if (__all_sync(0xffffffffu, wide_clear(g.ax.h, g.ay.h, i0, j0, nx, ny, 0, -1))) {
+        float ky[WV];
+        ik4(ky, g.ay.h.ik + j0);
+#pragma unroll
+        for (int r = 0; r < WR; ++r) {
+            const float kx = __ldg(g.ax.h.ik + i0 + r);
+#pragma unroll
+            for (int c = 0; c < WV; ++c) {
+                const float dyx = ey[r + 1][c] - ey[r][c],
+                            dxy = (c + 1 < WV ? ex[r][c + 1 < WV ? c + 1 : 0] : up[r]) - ex[r][c];
+                hz[r][c] = __fmaf_rn(-g.ch, __fsub_rn(__fmul_rn(dyx, kx), __fmul_rn(dxy, ky[c])), hz[r][c]);
+            }
+            st4(g.hz + o + (size_t)r * P, hz[r]);
+        }
+        return;
     }
     if (!col) return;
     const int wy = g.ay.h.lo + g.ay.h.hi;
@@ -483,7 +548,7 @@ __global__ void __launch_bounds__(32 * WT) tm2d_h_wide(const LensTM2D g) {
     }
 }
 
-__global__ void __launch_bounds__(32 * WT) tm2d_e_wide(const LensTM2D g, const int *rowref, const LensStepTable tab, int n) {
+__global__ void __launch_bounds__(32 * WT, WB) tm2d_e_wide(const LensTM2D g, const int *rowref, const LensStepTable tab, int n) {
     const int i0 = wide_i0(), j0 = wide_j0(), nx = g.nx, ny = g.ny, P = g.pitch;
     if (i0 >= nx) return;
     const bool col = j0 < ny, lossy = g.da_x != nullptr;
@@ -499,6 +564,33 @@ __global__ void __launch_bounds__(32 * WT) tm2d_e_wide(const LensTM2D g, const i
         ld4(ex[r], g.ex + o + (size_t)r * P, inx);
         ld4(ey[r], g.ey + o + (size_t)r * P, iny);
         dn[r] = wide_dn(hz[r + 1], g.hz + (size_t)i * P, j0, inx && j0 > 0);
+    }
+    if (__all_sync(0xffffffffu, wide_clear(g.ax.e, g.ay.e, i0, j0, nx, ny, 1, g.src.ix))) {
+        float ky[WV];
+        ik4(ky, g.ay.e.ik + j0);
+#pragma unroll
+        for (int r = 0; r < WR; ++r) {
+            const int i = i0 + r;
+            const size_t oc = (size_t)(rowref ? __ldg(rowref + i) : i) * P + j0;
+            float ca[WV], cb[WV], da[WV], db[WV];
+            ld4(ca, g.ca_x + oc, true);
+            ld4(cb, g.ca_y + oc, true);
+            if (lossy) {
+                ld4(da, g.da_x + oc, true);
+                ld4(db, g.da_y + oc, true);
+            }
+            const float kx = __ldg(g.ax.e.ik + i);
+#pragma unroll
+            for (int c = 0; c < WV; ++c) {
+                const float d = hz[r + 1][c] - (c > 0 ? hz[r + 1][c > 0 ? c - 1 : 0] : dn[r]), d2 = hz[r + 1][c] - hz[r][c];
+                const float e = lossy ? __fmul_rn(ex[r][c], da[c]) : ex[r][c], e2 = lossy ? __fmul_rn(ey[r][c], db[c]) : ey[r][c];
+                ex[r][c] = __fmaf_rn(ca[c], __fmul_rn(d, ky[c]), e);
+                ey[r][c] = __fmaf_rn(-cb[c], __fmul_rn(d2, kx), e2);
+            }
+            st4(g.ex + o + (size_t)r * P, ex[r]);
+            st4(g.ey + o + (size_t)r * P, ey[r]);
+        }
+        return;
     }
     if (!col) return;
     const int wy = g.ay.e.lo + g.ay.e.hi;
@@ -551,11 +643,47 @@ __global__ void __launch_bounds__(32 * WT) tm2d_e_wide(const LensTM2D g, const i
     }
 }
 
-// Epilogue of the new Ez after a wide E pass, blocks (bx0, by0) on of the grid.
+// Intensity on node (i, j) (fdtd2d_core.py:477-486), as the epilogues form it.
+__device__ __forceinline__ float node_inten(const LensTE2D &g, int i, int j) {
+    const float v = g.ez[(size_t)i * g.pitch + j];
+    return __fmul_rn(v, v);
+}
+
+__device__ __forceinline__ float node_inten(const LensTM2D &g, int i, int j) {
+    const float *ey = g.ey + (size_t)i * g.pitch, *ex = g.ex + (size_t)i * g.pitch + j;
+    const float f = j == 0 ? ey[0] : (j == g.ny - 1 ? ey[g.ny - 2] : 0.5f * (ey[j - 1] + ey[j]));
+    const float a = i > 0 ? ex[-g.pitch] : ex[0], b = i < g.nx - 1 ? ex[0] : a;
+    const float s2 = i == 0 || i == g.nx - 1 ? __fmul_rn(a, a) : 0.5f * __fmaf_rn(a, a, __fmul_rn(b, b));
+    return __fmaf_rn(f, f, s2);
+}
+
+// Detector boxes of a wide step that has no other epilogue: one launch for every box (z),
+// a block a tile of BX columns by 4 BY rows and one FP64 addition (the epilogue's one per
+// warp over two launches took 11 us each on boxes of 1600 x 80 nodes).
+constexpr int BOXR = 4;
+template <class G>
+__global__ void __launch_bounds__(BX *BY) box2d(const G g, const LensEpi2D ep) {
+    const int *bx = ep.box[blockIdx.z];
+    const int j = max(0, bx[2]) + blockIdx.x * BX + threadIdx.x, j1 = min(g.ny, bx[3]);
+    const int i0 = max(0, bx[0]) + (blockIdx.y * BY + threadIdx.y) * BOXR, i1 = min(g.nx, bx[1]);
+    double v = 0.0;
+#pragma unroll
+    for (int r = 0; r < BOXR; ++r)
+        if (j < j1 && i0 + r < i1) v += (double)node_inten(g, i0 + r, j);
+    __shared__ double red[BY];
+    v = warp_sum(v);
+    if (threadIdx.x == 0) red[threadIdx.y] = v;
+    __syncthreads();
+    if (threadIdx.y == 0) {
+        v = warp_sum(threadIdx.x < BY ? red[threadIdx.x] : 0.0);
+        if (threadIdx.x == 0 && v != 0.0) atomicAdd(ep.box_acc + blockIdx.z, v);
+    }
+}
+
+// Epilogue of the new Ez after a wide E pass.
 __global__ void __launch_bounds__(BX *BY)
-    te2d_epi(const LensTE2D g, const LensStepTable tab, const LensEpi2D ep, int n, int bx0, int by0) {
-    const int bx = blockIdx.x + bx0, by = blockIdx.y + by0;
-    const int j = bx * BX + threadIdx.x, i = by * BY + threadIdx.y;
+    te2d_epi(const LensTE2D g, const LensStepTable tab, const LensEpi2D ep, int n) {
+    const int j = blockIdx.x * BX + threadIdx.x, i = blockIdx.y * BY + threadIdx.y;
     const bool valid = i < g.nx && j < g.ny;
     const int P = g.pitch;
     const size_t o = (size_t)i * P + j;
@@ -566,7 +694,7 @@ __global__ void __launch_bounds__(BX *BY)
             for (int p = 0; p < ep.nplane; ++p)
                 if (i == ep.plane[p]) plane_node(ep, tab, n, p, P, j, ez, 0.5f * (g.hy[o - P] + g.hy[o]));
     }
-    epilogue_node(ep, tab, n, i, j, valid, o, ez, __fmul_rn(ez, ez), 0.f, bx, by);
+    epilogue_node(ep, tab, n, i, j, valid, o, ez, __fmul_rn(ez, ez), 0.f);
 }
 
 // Does the epilogue do more at step n than sum its boxes?
@@ -637,24 +765,14 @@ bool wide_ok(const LensEpi2D &e, const LensDrive2D *dr, std::initializer_list<co
     return true;
 }
 
-// Epilogue of a wide step: every block of the grid, or on steps that only sum boxes the
-// blocks of each box (run once with the other boxes' extents empty).
-template <class F>
-void wide_epilogue(const LensEpi2D &e, int n, int nx, int ny, F launch) {
-    if (epi2d_beyond_boxes(&e, n)) {
-        launch(e, 0, 0, (ny + BX - 1) / BX, (nx + BY - 1) / BY);
-        return;
-    }
+// Grid of box2d: the largest extents of the boxes, clipped to the grid (z: the box).
+dim3 box_grid(const LensEpi2D &e, int nx, int ny) {
+    int w = 0, h = 0;
     for (int b = 0; b < e.nbox; ++b) {
-        const int i0 = std::max(0, e.box[b][0]), i1 = std::min(nx, e.box[b][1]), j0 = std::max(0, e.box[b][2]),
-                  j1 = std::min(ny, e.box[b][3]);
-        if (i1 <= i0 || j1 <= j0) continue;
-        LensEpi2D one = e;
-        one.nbox = 1;
-        for (int q = 0; q < 4; ++q) one.box[0][q] = e.box[b][q];
-        one.box_acc = e.box_acc + b;
-        launch(one, j0 / BX, i0 / BY, (j1 + BX - 1) / BX - j0 / BX, (i1 + BY - 1) / BY - i0 / BY);
+        h = std::max(h, std::min(nx, e.box[b][1]) - std::max(0, e.box[b][0]));
+        w = std::max(w, std::min(ny, e.box[b][3]) - std::max(0, e.box[b][2]));
     }
+    return w > 0 && h > 0 ? dim3((w + BX - 1) / BX, (h + BY * BOXR - 1) / (BY * BOXR), e.nbox) : dim3(0, 1, 1);
 }
 
 int te2d_run(const LensTE2D *g, const LensStepTable *tab, const LensEpi2D *ep, const LensDrive2D *dr, int n0,
@@ -667,13 +785,12 @@ int te2d_run(const LensTE2D *g, const LensStepTable *tab, const LensEpi2D *ep, c
     cudaStream_t s = static_cast<cudaStream_t>(stream);
     const dim3 blk(BX, BY), grd((g->ny + BX - 1) / BX, (g->nx + BY - 1) / BY);
     if (wide_ok(e, dr, {g->ez, g->hx, g->hy, g->ce_e, g->ce_h})) {
-        const dim3 wb(BX, WT), wg((g->ny + BX * WV - 1) / (BX * WV), (g->nx + WT * WR - 1) / (WT * WR));
+        const dim3 wb(BX, WT), wg((g->ny + BX * WV - 1) / (BX * WV), (g->nx + WT * WR - 1) / (WT * WR)), bg = box_grid(e, g->nx, g->ny);
         for (int n = n0; n < n0 + nsteps; ++n) {
             te2d_h_wide<<<wg, wb, 0, s>>>(*g);
             te2d_e_wide<<<wg, wb, 0, s>>>(*g, rowref, *tab, n);
-            wide_epilogue(e, n, g->nx, g->ny, [&](const LensEpi2D &v, int bx, int by, int wx, int wy) {
-                te2d_epi<<<dim3(wx, wy), blk, 0, s>>>(*g, *tab, v, n, bx, by);
-            });
+            if (epi2d_beyond_boxes(&e, n)) te2d_epi<<<grd, blk, 0, s>>>(*g, *tab, e, n);
+            else if (bg.x > 0) box2d<<<bg, blk, 0, s>>>(*g, e);
         }
         return lens_cuda_status();
     }
@@ -695,20 +812,19 @@ int tm2d_run(const LensTM2D *g, const LensStepTable *tab, const LensEpi2D *ep, c
     cudaStream_t s = static_cast<cudaStream_t>(stream);
     const dim3 blk(BX, BY), grd((g->ny + BX - 1) / BX, (g->nx + BY - 1) / BY);
     if (wide_ok(e, dr, {g->ex, g->ey, g->hz, g->ca_x, g->ca_y, g->da_x, g->da_y})) {
-        const dim3 wb(BX, WT), wg((g->ny + BX * WV - 1) / (BX * WV), (g->nx + WT * WR - 1) / (WT * WR));
+        const dim3 wb(BX, WT), wg((g->ny + BX * WV - 1) / (BX * WV), (g->nx + WT * WR - 1) / (WT * WR)), bg = box_grid(e, g->nx, g->ny);
         for (int n = n0; n < n0 + nsteps; ++n) {
             tm2d_h_wide<<<wg, wb, 0, s>>>(*g);
             tm2d_e_wide<<<wg, wb, 0, s>>>(*g, rowref, *tab, n);
-            wide_epilogue(e, n, g->nx, g->ny, [&](const LensEpi2D &v, int bx, int by, int wx, int wy) {
-                tm2d_epi<<<dim3(wx, wy), blk, 0, s>>>(*g, *tab, v, n, bx, by);
-            });
+            if (epi2d_beyond_boxes(&e, n)) tm2d_epi<<<grd, blk, 0, s>>>(*g, *tab, e, n);
+            else if (bg.x > 0) box2d<<<bg, blk, 0, s>>>(*g, e);
         }
         return lens_cuda_status();
     }
     for (int n = n0; n < n0 + nsteps; ++n) {
         tm2d_h<<<grd, blk, 0, s>>>(*g);
         tm2d_e<<<grd, blk, 0, s>>>(*g, *tab, n, d);
-        if (epi2d_active(&e, n)) tm2d_epi<<<grd, blk, 0, s>>>(*g, *tab, e, n, 0, 0);
+        if (epi2d_active(&e, n)) tm2d_epi<<<grd, blk, 0, s>>>(*g, *tab, e, n);
     }
     return lens_cuda_status();
 }
