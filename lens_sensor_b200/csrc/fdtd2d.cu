@@ -757,7 +757,14 @@ bool drive2d_ok(const LensDrive2D *d, const LensStepTable *tab, int nx) {
 }
 
 // The wide passes carry every plain step whose arrays start on 16-byte boundaries; the
-// stitch drive, the stitch sums and the pulse planes stay with one cell a thread.
+// stitch drive, the stitch sums and the pulse planes stay with one cell a thread.  A small
+// grid's passes last as long as one warp, and a wide one does eight times the work, half of
+// it in strips: us a step, one cell a thread / wide, TM 20.6 / 22.7 on 4000 x 128 cells and
+// 27.7 / 22.7 on 4000 x 200; TE with boxes 22.5 / 22.7 on 4000 x 256 and 26.5 / 24.0 on 4000 x
+// 300; TE inside its DFT windows, which the one-cell pass sums while it holds the field,
+// 34.9 / 39.3 on 4000 x 300 and 62.6 / 61.0 on 4000 x 500.
+constexpr double WIDE_TM = 0.7e6, WIDE_TE = 1.1e6, WIDE_TE_WINDOW = 1.9e6;  // cells
+
 bool wide_ok(const LensEpi2D &e, const LensDrive2D *dr, std::initializer_list<const void *> arrays) {
     if (dr || e.nsx > 0 || e.dft_raw || e.ex2) return false;
     for (const void *p : arrays)
@@ -784,10 +791,15 @@ int te2d_run(const LensTE2D *g, const LensStepTable *tab, const LensEpi2D *ep, c
     const LensDrive2D d = dr ? *dr : LensDrive2D{};
     cudaStream_t s = static_cast<cudaStream_t>(stream);
     const dim3 blk(BX, BY), grd((g->ny + BX - 1) / BX, (g->nx + BY - 1) / BY);
-    if (wide_ok(e, dr, {g->ez, g->hx, g->hy, g->ce_e, g->ce_h})) {
+    const double cells = (double)g->nx * g->ny;
+    if (cells >= WIDE_TE && wide_ok(e, dr, {g->ez, g->hx, g->hy, g->ce_e, g->ce_h})) {
         const dim3 wb(BX, WT), wg((g->ny + BX * WV - 1) / (BX * WV), (g->nx + WT * WR - 1) / (WT * WR)), bg = box_grid(e, g->nx, g->ny);
         for (int n = n0; n < n0 + nsteps; ++n) {
             te2d_h_wide<<<wg, wb, 0, s>>>(*g);
+            if (cells < WIDE_TE_WINDOW && epi2d_beyond_boxes(&e, n)) {
+                te2d_e<<<grd, blk, 0, s>>>(*g, *tab, e, n, d);
+                continue;
+            }
             te2d_e_wide<<<wg, wb, 0, s>>>(*g, rowref, *tab, n);
             if (epi2d_beyond_boxes(&e, n)) te2d_epi<<<grd, blk, 0, s>>>(*g, *tab, e, n);
             else if (bg.x > 0) box2d<<<bg, blk, 0, s>>>(*g, e);
@@ -811,7 +823,7 @@ int tm2d_run(const LensTM2D *g, const LensStepTable *tab, const LensEpi2D *ep, c
     const LensDrive2D d = dr ? *dr : LensDrive2D{};
     cudaStream_t s = static_cast<cudaStream_t>(stream);
     const dim3 blk(BX, BY), grd((g->ny + BX - 1) / BX, (g->nx + BY - 1) / BY);
-    if (wide_ok(e, dr, {g->ex, g->ey, g->hz, g->ca_x, g->ca_y, g->da_x, g->da_y})) {
+    if ((double)g->nx * g->ny >= WIDE_TM && wide_ok(e, dr, {g->ex, g->ey, g->hz, g->ca_x, g->ca_y, g->da_x, g->da_y})) {
         const dim3 wb(BX, WT), wg((g->ny + BX * WV - 1) / (BX * WV), (g->nx + WT * WR - 1) / (WT * WR)), bg = box_grid(e, g->nx, g->ny);
         for (int n = n0; n < n0 + nsteps; ++n) {
             tm2d_h_wide<<<wg, wb, 0, s>>>(*g);

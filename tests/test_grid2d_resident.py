@@ -171,9 +171,11 @@ def test_watchdog_ends_the_launch():
     assert bool(torch.isfinite(a.ez).all())
 
 
-WIDE = [('s', 60, 33, False, {}), ('p', 61, 65, True, {}), ('p', 133, 128, False, {}), ('s', 301, 257, False, {}),
-        ('p', 300, 700, True, {}), ('s', 97, 131, False, dict(full_x=True)), ('p', 90, 70, True, dict(source=False)),
-        ('s', 64, 100, False, dict(pec=(0, 1, 0, 1))), ('p', 65, 100, True, dict(pec=(1, 0, 1, 0)))]
+WIDE = [  # from the size the wide passes start at
+    ('s', 8200, 257, False, {}), ('s', 3001, 401, False, {}), ('s', 16001, 130, False, {}), ('p', 2701, 263, True, {}),
+    ('p', 5501, 128, False, {}), ('p', 1030, 700, True, {}), ('s', 4100, 513, False, dict(full_x=True)),
+    ('p', 2700, 301, True, dict(source=False)), ('s', 4101, 500, False, dict(pec=(0, 1, 0, 1))),
+    ('p', 2703, 300, True, dict(pec=(1, 0, 1, 0)))]
 
 
 @pytest.mark.gpu
@@ -185,7 +187,7 @@ def test_wide_passes_keep_the_bits(case, rows, monkeypatch):
     import torch
     from lens_sensor_b200 import engine as E
     pol, nx, ny, lossy, kw = case
-    steps = 12
+    steps = 8
     a, b = (_grid(pol, nx, ny, lossy, 9, **kw) for _ in range(2))
     monkeypatch.setattr(E, 'RS_MIN_STEPS', 1 << 30)
     if rows:
