@@ -1307,6 +1307,74 @@ __global__ void __launch_bounds__(NT) accum_e2(const K3 g, int target, int nxt, 
     iavg[((size_t)i * ny + j) * P + k] += (a + b) + d;
 }
 
+// The same with four z cells per thread: a thread reads each row it averages once, as 16
+// bytes and the one value beyond them that a z shift needs, instead of up to nine scattered
+// loads a cell with every index clamped anew (100 us on 301 x 141 x 203 cells; reading each
+// field and the average once is 29 us of the measured copy rate).  Needs 16-byte aligned arrays.
+constexpr int AV = 4;
+
+// Squares of row (i, j) of F averaged over x as sqx does, for k0-1 .. k0+AV (entries 0 .. AV+1;
+// lo / hi: is the entry before / beyond the four read?).
+__device__ __forceinline__ void sq_row(float (&o)[AV + 2], const float *F, const Ext &f, int tnx, int P, int ny, int i, int j,
+                                       int k0, bool lo, bool hi) {
+    const bool two = f.nx != tnx;
+    const int i0 = two ? min(max(i - 1, 0), f.nx - 1) : i, i1 = two ? min(max(i, 0), f.nx - 1) : i;
+    const float *p = F + ((size_t)i0 * ny + j) * P + k0, *q = F + ((size_t)i1 * ny + j) * P + k0;
+    const float4 a = *reinterpret_cast<const float4 *>(p), b = two ? *reinterpret_cast<const float4 *>(q) : a;
+    const float x[AV + 2] = {lo ? p[-1] : 0.f, a.x, a.y, a.z, a.w, hi ? p[AV] : 0.f};
+    const float y[AV + 2] = {lo ? (two ? q[-1] : x[0]) : 0.f, b.x, b.y, b.z, b.w, hi ? (two ? q[AV] : x[AV + 1]) : 0.f};
+#pragma unroll
+    for (int c = 0; c < AV + 2; ++c) o[c] = two ? 0.5f * (x[c] * x[c] + y[c] * y[c]) : x[c] * x[c];
+}
+
+__device__ __forceinline__ void sq4_on_grid(float (&o)[AV], const float *F, const Ext &f, const Ext &t, int P, int ny, int i,
+                                            int j, int k0) {
+    const bool longer = f.nz == t.nz + 1, shorter = f.nz == t.nz - 1;
+    const bool lo = shorter && k0 > 0, hi = longer && k0 + AV < f.nz;
+    // y rows: the component's own, j and j+1 of a longer one, j-1 and j of a shorter one (edges copied)
+    int j0 = j, j1 = j;
+    if (f.ny == t.ny + 1) j1 = j + 1;
+    else if (f.ny != t.ny) {
+        j0 = j == 0 ? 0 : j - 1;
+        j1 = j == t.ny - 1 ? f.ny - 1 : (j == 0 ? 0 : j);
+        if (j == t.ny - 1) j0 = j1;
+    }
+    float u[AV + 2];
+    sq_row(u, F, f, t.nx, P, ny, i, j0, k0, lo, hi);
+    if (j1 != j0) {
+        float v[AV + 2];
+        sq_row(v, F, f, t.nx, P, ny, i, j1, k0, lo, hi);
+#pragma unroll
+        for (int c = 0; c < AV + 2; ++c) u[c] = 0.5f * (u[c] + v[c]);
+    }
+#pragma unroll
+    for (int c = 0; c < AV; ++c) {
+        const int k = k0 + c;
+        if (longer) o[c] = 0.5f * (u[c + 1] + u[c + 2]);
+        else if (shorter) o[c] = k == 0 ? u[c + 1] : (k == t.nz - 1 ? u[c] : 0.5f * (u[c] + u[c + 1]));
+        else o[c] = u[c + 1];
+    }
+}
+
+__global__ void __launch_bounds__(NT) accum_e2v(const K3 g, int target, int nxt, float *iavg) {
+    const int k0 = (blockIdx.x * BK + threadIdx.x) * AV, j = blockIdx.y * BJ + threadIdx.y, i = blockIdx.z;
+    const int ny = g.ny, nz = g.nz, P = g.P;
+    const Ext ex{nxt - 1, ny, nz}, ey{nxt, ny - 1, nz}, ez{nxt, ny, nz - 1};
+    const Ext t = target == 1 ? ey : ez;
+    if (i >= t.nx || j >= t.ny || k0 >= t.nz) return;
+    float a[AV], b[AV], d[AV];
+    float4 *acc = reinterpret_cast<float4 *>(iavg + ((size_t)i * ny + j) * P + k0);
+    float4 s = *acc;
+    sq4_on_grid(a, g.ex, ex, t, P, ny, i, j, k0);
+    sq4_on_grid(b, g.ey, ey, t, P, ny, i, j, k0);
+    sq4_on_grid(d, g.ez, ez, t, P, ny, i, j, k0);
+    s.x += (a[0] + b[0]) + d[0];  // the cells beyond t.nz keep what they hold
+    if (k0 + 1 < t.nz) s.y += (a[1] + b[1]) + d[1];
+    if (k0 + 2 < t.nz) s.z += (a[2] + b[2]) + d[2];
+    if (k0 + 3 < t.nz) s.w += (a[3] + b[3]) + d[3];
+    *acc = s;
+}
+
 // ============================================================ host side
 bool ax_ok(const LensAxis &a, int n) { return lens_profile_ok(a.e, n) && lens_profile_ok(a.h, n - 1); }
 
@@ -1701,6 +1769,13 @@ extern "C" int lens_fdtd3d_accum_e2(const LensGrid3D *g, int target, int nx_targ
     if (!grid3d_ok(g) || !iavg || (target != 1 && target != 2) || nx_target < 2 || nx_target > g->nx)
         return LENS_ERR_ARG;
     const dim3 blk(BK, BJ), grd(g->pitch / BK, (g->ny + BJ - 1) / BJ, nx_target);
+    bool al = (reinterpret_cast<uintptr_t>(iavg) & 15) == 0;
+    for (int c = 0; c < 3; ++c) al = al && (reinterpret_cast<uintptr_t>(g->f[g->cur][c]) & 15) == 0;
+    if (al) {
+        accum_e2v<<<dim3((g->pitch + BK * AV - 1) / (BK * AV), grd.y, nx_target), blk, 0, static_cast<cudaStream_t>(stream)>>>(
+            view(g, g->cur, g->cur), target, nx_target, iavg);
+        return lens_cuda_status();
+    }
     accum_e2<<<grd, blk, 0, static_cast<cudaStream_t>(stream)>>>(view(g, g->cur, g->cur), target, nx_target,
                                                                   iavg);
     return lens_cuda_status();
