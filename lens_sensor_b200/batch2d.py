@@ -42,13 +42,25 @@ def row_types(arrays, shape, dev, min_rows=8):
     rows) whose rows form the table (ntype, ncoef, pitch).  Returns (None, None)
     when no group qualifies."""
     nx, P = shape
-    a = np.zeros((nx, len(arrays), P), np.float32)
-    for q, v in enumerate(arrays):
-        v = np.asarray(v, np.float32)
-        a[:v.shape[0], q, :v.shape[1]] = v
+    arrays = [np.ascontiguousarray(v, np.float32) for v in arrays]
+    new = np.zeros(nx, bool)      # rows that differ from the row before: equal rows come in runs
+    new[0] = True
+    for v in arrays:
+        b = v.view(np.int32)
+        new[1:v.shape[0]] |= (b[1:] != b[:-1]).any(axis=1)
+        if v.shape[0] < nx:
+            new[v.shape[0]] = True
+
+    def row(i):
+        r = np.zeros((len(arrays), P), np.float32)
+        for q, v in enumerate(arrays):
+            if i < v.shape[0]:
+                r[q, :v.shape[1]] = v[i]
+        return r
     groups = {}
-    for i in range(nx):
-        groups.setdefault(a[i].tobytes(), []).append(i)
+    heads = np.flatnonzero(new)
+    for i, j in zip(heads, np.append(heads[1:], nx)):
+        groups.setdefault(row(i).tobytes(), []).extend(range(i, j))
     best = sorted(groups.values(), key=len, reverse=True)[:MAX_RTYPE]
     best = [g for g in best if len(g) >= min_rows]
     if not best:
@@ -57,7 +69,7 @@ def row_types(arrays, shape, dev, min_rows=8):
     tab = np.zeros((len(best), len(arrays), P), np.float32)
     for t, g in enumerate(best):
         rt[g] = t
-        tab[t] = a[g[0]]
+        tab[t] = row(g[0])
     return torch.from_numpy(rt).to(dev), torch.from_numpy(tab).to(dev)
 
 
