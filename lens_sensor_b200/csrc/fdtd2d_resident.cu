@@ -119,15 +119,27 @@ __device__ __forceinline__ float opaque_zero() {
     return z;
 }
 
-__device__ __forceinline__ void dft_add(float *dft, bool kahan, size_t o, float v, float pr, float pim) {
+// Node DFT of two rows' values at offset o (the second P nodes on, if on1): both rows'
+// sums are loaded before the first is stored.  One by one the compiler kept every load
+// behind the store before it, an L2 round trip a row; more rows together spill.
+__device__ __forceinline__ void dft_add2(float *dft, bool kahan, size_t o, int P, bool on1, float v0, float v1, float pr,
+                                         float pim) {
     if (kahan) {
-        kahan_add(reinterpret_cast<float4 *>(dft) + o, v * pr, v * pim);
+        float4 *a = reinterpret_cast<float4 *>(dft) + o;
+        float4 s0 = a[0], s1 = on1 ? a[P] : s0;
+        kahan_reg(s0, v0 * pr, v0 * pim);
+        kahan_reg(s1, v1 * pr, v1 * pim);
+        a[0] = s0;
+        if (on1) a[P] = s1;
     } else {
         float2 *a = reinterpret_cast<float2 *>(dft) + o;
-        float2 s = *a;
-        s.x += v * pr;
-        s.y += v * pim;
-        *a = s;
+        float2 s0 = a[0], s1 = on1 ? a[P] : s0;
+        s0.x = __fmaf_rn(v0, pr, s0.x);
+        s0.y = __fmaf_rn(v0, pim, s0.y);
+        s1.x = __fmaf_rn(v1, pr, s1.x);
+        s1.y = __fmaf_rn(v1, pim, s1.y);
+        a[0] = s0;
+        if (on1) a[P] = s1;
     }
 }
 
@@ -578,8 +590,9 @@ __device__ __forceinline__ void rs_band(const LensInst2D *__restrict__ insts, co
         if (POL == 0 && win && (tf & T_JLT)) {  // node DFT of Ez
             const float pr = __ldg(tab.pe + 2 * k), pim = __ldg(tab.pe + 2 * k + 1);
 #pragma unroll
-            for (int r = 0; r < RM; ++r)
-                if (r < R) dft_add(B.dft, bf & B_KAHAN, (size_t)(B.lo + r) * B.P + j, fa[r], pr, pim);
+            for (int r = 0; r < RM; r += 2)
+                if (r < R) dft_add2(B.dft, bf & B_KAHAN, (size_t)(B.lo + r) * B.P + j, B.P, r + 1 < R, fa[r],
+                                    fa[r + 1 < RM ? r + 1 : r], pr, pim);
         }
         if (B.frames && (m + 1) % B.every == 0 && (m + 1) / B.every <= B.nframes) {
             const int nyf = POL == 0 ? ny : ny - 1;
@@ -598,14 +611,14 @@ __device__ __forceinline__ void rs_band(const LensInst2D *__restrict__ insts, co
         if (POL == 1 && win) {  // TM node DFT: Ey averaged onto the nodes (fdtd2d_core.py:458-465)
             const float pr = __ldg(tab.pe + 2 * k), pim = __ldg(tab.pe + 2 * k + 1);
 #pragma unroll
-            for (int r = 0; r < RM; ++r) {
+            for (int r = 0; r < RM; r += 2) {
                 if (r < R) {
-                    const float ey = fb[r];
-                    const float eyl = nb_dn(eb, ey, r);
-                    if (tf & T_JLT) {
-                        const float v = j == 0 ? ey : (j == ny - 1 ? eyl : 0.5f * (eyl + ey));
-                        dft_add(B.dft, bf & B_KAHAN, (size_t)(B.lo + r) * B.P + j, v, pr, pim);
-                    }
+                    const float e0 = fb[r], e1 = fb[r + 1 < RM ? r + 1 : r];
+                    const float l0 = nb_dn(eb, e0, r), l1 = nb_dn(eb, e1, r + 1 < RM ? r + 1 : r);
+                    const float v0 = j == 0 ? e0 : (j == ny - 1 ? l0 : 0.5f * (l0 + e0));
+                    const float v1 = j == 0 ? e1 : (j == ny - 1 ? l1 : 0.5f * (l1 + e1));
+                    if (tf & T_JLT)
+                        dft_add2(B.dft, bf & B_KAHAN, (size_t)(B.lo + r) * B.P + j, B.P, r + 1 < R, v0, v1, pr, pim);
                 }
             }
         }
