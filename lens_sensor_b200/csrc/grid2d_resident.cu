@@ -43,7 +43,8 @@ size_t rs_smem(const RsForm &f, int ncol, int nc, int nbox, bool hold) {
 }
 
 // Relative cost of a row and, in percent of its bands' cost, what a further CTA on an SM
-// adds to a step (1600 x 384 cells: 1.95 us with two CTAs of 6 rows, 2.4 with one of 12).
+// adds to a step: CTAs on an SM overlap one's halo wait with another's rows, so two bands of
+// half the rows cost more than one of them and less than both in turn.
 constexpr int RS_COST_LEAN = 10, RS_COST_SPECIAL = 34, RS_SHARE = 30;
 
 // Runs of special and of other rows of a grid, in order.

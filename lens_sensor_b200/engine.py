@@ -197,7 +197,9 @@ class Grid2D:
                             _ptr(self.psi['hzx']), _ptr(self.psi['hzy']), _ptr(self.psi['exy']),
                             _ptr(self.psi['eyx']), pec4, s)
 
-        # scratch and error word of the resident launch (lens_te2d_resident), when the grid fits the chip
+        # scratch and error word of the resident launch (lens_te2d_resident), when the grid fits the chip;
+        # launches step() has made (a resident launch once per call, the passes H and E once per step)
+        self.launches = 0
         need = (self.lib.lens_te2d_resident_bytes if self.pol == 's' else self.lib.lens_tm2d_resident_bytes)(
             ctypes.byref(self.s))
         self.rs_scratch = torch.empty(need, dtype=torch.uint8, device=dev) if need else None
@@ -236,7 +238,9 @@ class Grid2D:
             st = fn(ctypes.byref(self.s), ctypes.byref(table.s), e, int(n0), int(nsteps), _ptr(self.rs_scratch),
                     self.rs_scratch.numel(), _ptr(self.rs_err), _stream_ptr(stream))
             if st != N.ERR_SIZE:      # else: a call that only the steps below carry
+                self.launches += 1
                 return N.check(st)
+        self.launches += 2 * max(0, int(nsteps))
         if drive is None:
             fn = self.lib.lens_te2d_step_rows if self.pol == 's' else self.lib.lens_tm2d_step_rows
             N.check(fn(ctypes.byref(self.s), _ptr(self.rowref), ctypes.byref(table.s), e, int(n0), int(nsteps),
@@ -245,7 +249,6 @@ class Grid2D:
             fn = self.lib.lens_te2d_step_driven if self.pol == 's' else self.lib.lens_tm2d_step_driven
             N.check(fn(ctypes.byref(self.s), ctypes.byref(table.s), e, ctypes.byref(drive.s), int(n0),
                        int(nsteps), _stream_ptr(stream)))
-
 
     def check(self):
         """Raise if a resident launch's wait between bands ran out (the fields hold NaN then)."""

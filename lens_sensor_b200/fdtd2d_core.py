@@ -235,6 +235,7 @@ def run_beads(wg_mat, bead_mat, bead_d_um, dx_nm=20.0, save_frames=True, n_snaps
                 ep.restart_dft((steps_total, steps_total + n_acc))
                 nacc_prev = n_acc
                 steps_total += n_acc
+    _check(g)
     if ez_mm is not None:
         ez_mm.flush()
         del ez_mm
@@ -776,6 +777,7 @@ def run_beads_sliding(wg_mat, bead_mat, bead_d_um, dx_nm, save_frames, n_snapsho
                                'y_end': (y0_m + H_total) * 1e6, 'slide_i': slide_i, 'step': n,
                                'time': time.time() - t_start})
                 k_fr += 1
+        _check(grid)
         box = ep.box_acc.double().cpu().numpy()
         for q, which in enumerate(names):
             sums[which + '_P'] += float(box[q])
@@ -832,6 +834,12 @@ class FluxSum2D:
         if not self.has(key):
             return float('nan')
         return self.E.plane_flux(self.acc[key], self.n[key])
+
+
+def _check(grid):
+    """Raise if a launch of the grid's steps reported an error (a grid that can tell)."""
+    if hasattr(grid, 'check'):
+        grid.check()
 
 
 def _field_2d(g):

@@ -61,8 +61,10 @@ class Solve2D:
     replays); engine='tb': the temporally blocked step (lens_tb2d_step,
     LENS_TB_K steps per launch; the schedule and the snapshot period must be
     whole numbers of launch pairs; chunk: rows per warp); engine='step': the
-    single-grid engine (lens_te2d_step / lens_tm2d_step), one step per launch
-    pair, with the full single-grid epilogue set."""
+    single-grid engine with the full single-grid epilogue set: one cooperative
+    launch per snapshot period when the grid fits the chip (lens_te2d_resident /
+    lens_tm2d_resident), else one step per launch pair (lens_te2d_step /
+    lens_tm2d_step)."""
 
     def __init__(self, spec: Spec2D, steps_total, periods=1, snap_every=200, device=None, geo=None, engine=None,
                  chunk=16, by=4):
@@ -131,8 +133,9 @@ class Solve2D:
             self.launches += 1
             return
         if self.engine == 'step':
+            l0 = self.grid.launches
             self.grid.step(self.table, n, m - n, self.epi, stream)
-            self.launches += 2 * (m - n)
+            self.launches += self.grid.launches - l0
             return
         if self.engine == 'persistent':
             self.group.step_persistent(self.table, n, m - n, stream)
@@ -191,6 +194,8 @@ class Solve2D:
         """Raise if a resident launch's wait between bands ran out."""
         if self.engine == 'resident':
             self.group.check()
+        elif self.engine == 'step':
+            self.grid.check()
 
     def phasor(self):
         """(2/N) sum F e^{-i w t} on the nodes (nx, ny), complex128 on the device."""
