@@ -75,8 +75,11 @@ def repeated_rows(arrays):
     return torch.cummax(torch.where(new, idx, torch.zeros_like(idx)), dim=0).values.to(torch.int32)
 
 
-# Steps from which Grid2D.step takes the resident launch: a launch of few steps pays for
-# the state's way in and out (see the launch in csrc/grid2d_resident.cuh).
+# Steps from which Grid2D.step takes the resident launch, which pays for the state's way in
+# and out: us a call, resident / step by step, at 3 and at 4 steps: TE 140 x 96 with boxes
+# 37.6 / 43.2 and 39.0 / 50.2, TE 1600 x 480 with boxes 64.4 / 64.8 and 66.3 / 83.1, TM 1201 x
+# 431 with every epilogue 96.8 / 89.0 and 108.6 / 115.7, TE 1201 x 431 75.6 / 65.1 and 83.6 /
+# 83.3 (at 1 step 61 / 29, at 16 steps 156 / 306).
 RS_MIN_STEPS = 4
 
 
@@ -204,9 +207,15 @@ class Grid2D:
             ctypes.byref(self.s))
         self.rs_scratch = torch.empty(need, dtype=torch.uint8, device=dev) if need else None
         self.rs_err = torch.zeros(1, dtype=torch.int32, device=dev) if need else None
-        # coefficient rows that repeat, read once by the step by step passes of a grid beyond the chip
-        self.rowref = None if need else repeated_rows(
-            [self.ce_e, self.ce_h] if self.pol == 's' else [self.ca_x, self.ca_y] + ([self.da_x, self.da_y] if da else []))
+        # coefficient rows that repeat, read once by the step by step passes of a grid beyond the chip,
+        # while the coefficients stay as they were given (the arrays' version counters tell)
+        self._coef = [a for a in ([self.ce_e, self.ce_h] if self.pol == 's' else
+                                  [self.ca_x, self.ca_y, self.da_x, self.da_y]) if a is not None]
+        self._coef_version = self._versions()
+        self.rowref = None if need or self._coef_version is None else repeated_rows(self._coef)
+
+    def _versions(self):
+        return None if any(a.is_inference() for a in self._coef) else [a._version for a in self._coef]
 
     # reference-shaped views of the resident fields
     def view(self, name):
@@ -243,7 +252,8 @@ class Grid2D:
         self.launches += 2 * max(0, int(nsteps))
         if drive is None:
             fn = self.lib.lens_te2d_step_rows if self.pol == 's' else self.lib.lens_tm2d_step_rows
-            N.check(fn(ctypes.byref(self.s), _ptr(self.rowref), ctypes.byref(table.s), e, int(n0), int(nsteps),
+            rows = self.rowref if self.rowref is not None and self._versions() == self._coef_version else None
+            N.check(fn(ctypes.byref(self.s), _ptr(rows), ctypes.byref(table.s), e, int(n0), int(nsteps),
                        _stream_ptr(stream)))
         else:
             fn = self.lib.lens_te2d_step_driven if self.pol == 's' else self.lib.lens_tm2d_step_driven

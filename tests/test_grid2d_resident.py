@@ -214,3 +214,20 @@ def test_wide_passes_keep_the_bits(case, rows, monkeypatch):
     for q in ('box_acc', 'plane_acc'):
         x, y = getattr(ea, q), getattr(eb, q)
         assert float((x - y).abs().max()) <= 1e-12 * max(float(y.abs().max()), 1e-300), q
+
+
+@pytest.mark.gpu
+def test_coefficients_written_in_place():
+    """A large grid whose coefficients change after it was made steps with the new ones."""
+    import torch
+    from lens_sensor_b200 import engine as E
+    a, b = (_grid('s', 3001, 401, False, 9) for _ in range(2))
+    assert a.rowref is not None
+    for g in (a, b):
+        g.ce_e[1400:1500].mul_(0.75)
+    tab = E.StepTable(7, 8, a.dt, 2.2e15, 2.2e15, E.cw_envelope(3.5e14))
+    a.step(tab, 7, 8)
+    assert b.lib.lens_te2d_step(ctypes.byref(b.s), ctypes.byref(tab.s), None, 7, 8, None) == 0
+    torch.cuda.synchronize()
+    for q in FIELDS['s']:
+        assert torch.equal(getattr(a, q), getattr(b, q)), q
