@@ -643,6 +643,79 @@ __global__ void __launch_bounds__(32 * WT, WB) tm2d_e_wide(const LensTM2D g, con
     }
 }
 
+// ---- coefficient rows that repeat
+// For every row the first row of the run of rows it lies in that hold the same bits in
+// every coefficient array.  Formed anew by each call that steps with it, from the
+// coefficients as they are then: nothing of it outlives the call.
+struct RowArrays {
+    const float *a[4];
+    int rows[4];  // rows that the array's component has (the last one of an x component is never compared)
+    int n;
+};
+constexpr int RRB = 8, RRT = 128;  // rows, threads of a block
+
+// ref[i] = i where row i differs from the row before, else 0.  Reads every coefficient
+// once (and one row in eight again, from the caches): bound by memory, 47 us for the four
+// arrays of 16000 x 700 TM cells between steps (179 MB, 3.8 TB/s).  Called over and over, part
+// of them in the L2, 35 us, and 42 / 38 at 4 / 16 rows a block, 39 at 256 threads.
+__global__ void __launch_bounds__(RRT) row_heads(const RowArrays v, int nx, int ny, int P, int *ref) {
+    const int i0 = blockIdx.x * RRB, q4 = (ny + 3) / 4;
+    unsigned diff = 0;
+    for (int m = threadIdx.x; m < v.n * q4; m += RRT) {
+        const int q = m / q4, rows = v.rows[q];
+        const float *a = v.a[q] + 4 * (m - q * q4);
+        int4 b[RRB + 1];
+#pragma unroll
+        for (int r = 0; r <= RRB; ++r)  // rows beyond the array: its last again
+            b[r] = __ldg(reinterpret_cast<const int4 *>(a + (size_t)min(max(i0 + r - 1, 0), rows - 1) * P));
+#pragma unroll
+        for (int r = 0; r < RRB; ++r)
+            diff |= (((b[r].x ^ b[r + 1].x) | (b[r].y ^ b[r + 1].y) | (b[r].z ^ b[r + 1].z) | (b[r].w ^ b[r + 1].w)) != 0 ? 1u : 0u) << r;
+    }
+    __shared__ unsigned all;
+    if (threadIdx.x == 0) all = 0;
+    __syncthreads();
+    diff = __reduce_or_sync(0xffffffffu, diff);
+    if ((threadIdx.x & 31) == 0 && diff) atomicOr(&all, diff);
+    __syncthreads();
+    const int r = threadIdx.x;
+    if (r < RRB && i0 + r < nx) ref[i0 + r] = (all >> r & 1u) ? i0 + r : 0;
+}
+
+// The last row at or before each that row_heads marked, in place: one block, a warp 32
+// rows at a time (a ballot names their heads), its RRN groups loaded before any is looked at.
+// Bound by one SM's latency: 16000 rows 14.7 us with RRN neighbouring rows a thread, 5.1 here.
+constexpr int RRS = 1024, RRN = 16;
+__global__ void __launch_bounds__(RRS) row_runs(int *ref, int nx) {
+    __shared__ int part[RRS / 32];
+    const int lane = threadIdx.x & 31, w = threadIdx.x / 32;
+    int before = 0;  // last head of the rounds before
+    for (int base = 0; base < nx; base += RRS * RRN) {
+        const int i0 = base + w * 32 * RRN;
+        int v[RRN], last = -1;  // last head of this warp's rows
+#pragma unroll
+        for (int q = 0; q < RRN; ++q) v[q] = i0 + 32 * q + lane < nx ? ref[i0 + 32 * q + lane] : 0;
+#pragma unroll
+        for (int q = 0; q < RRN; ++q) {
+            const unsigned heads = __ballot_sync(0xffffffffu, v[q] != 0), m = heads & (0xffffffffu >> (31 - lane));
+            v[q] = m ? i0 + 32 * q + 31 - __clz(m) : last;
+            if (heads) last = i0 + 32 * q + 31 - __clz(heads);
+        }
+        if (lane == 0) part[w] = last;
+        __syncthreads();
+        int run = before;
+#pragma unroll
+        for (int q = 0; q < RRS / 32; ++q) {
+            if (q < w) run = max(run, part[q]);
+            before = max(before, part[q]);
+        }
+        __syncthreads();
+#pragma unroll
+        for (int q = 0; q < RRN; ++q)
+            if (i0 + 32 * q + lane < nx) ref[i0 + 32 * q + lane] = v[q] >= 0 ? v[q] : run;
+    }
+}
+
 // Intensity on node (i, j) (fdtd2d_core.py:477-486), as the epilogues form it.
 __device__ __forceinline__ float node_inten(const LensTE2D &g, int i, int j) {
     const float v = g.ez[(size_t)i * g.pitch + j];
@@ -772,6 +845,28 @@ bool wide_ok(const LensEpi2D &e, const LensDrive2D *dr, std::initializer_list<co
     return true;
 }
 
+// A span forms a row table where the coefficients come from memory, not from the L2 (126
+// MB): by the bytes of fields and coefficients.  us a step without / with the table: TM 1600 x
+// 480 to 4000 x 448 cells (50 MB) the same within 0.5 %, 4000 x 700 (79 MB) 36.1 / 33.3, 16000 x
+// 200 (100 MB) 61.9 / 51.3, 8000 x 700 (158 MB) 69.9 / 49.9, 16000 x 700 (315 MB) 122.8 / 105.7;
+// TE 16000 x 200 (72 MB) 47.0 / 46.6, 8000 x 700 (113 MB) 51.9 / 43.1, 16000 x 700 (225 MB) 102.4
+// / 95.0.  Forming it takes 19 to 52 us, two to four steps' gain; a grid without repeated
+// rows loses that, 5 % of the shortest span that forms one.  (Formed once with the grid and
+// kept, the table went stale when the coefficients were written past its check.)
+constexpr double ROW_BYTES = 90e6;
+constexpr int ROW_STEPS = 8;
+
+bool row_table_pays(int nx, int P, int arrays, int nsteps) {
+    return nsteps >= ROW_STEPS && 4.0 * nx * P * arrays >= ROW_BYTES;
+}
+
+int row_table(const RowArrays &v, int nx, int ny, int P, int *rowref, void *stream) {
+    cudaStream_t s = static_cast<cudaStream_t>(stream);
+    row_heads<<<(nx + RRB - 1) / RRB, RRT, 0, s>>>(v, nx, ny, P, rowref);
+    row_runs<<<1, RRS, 0, s>>>(rowref, nx);
+    return lens_cuda_status();
+}
+
 // Grid of box2d: the largest extents of the boxes, clipped to the grid (z: the box).
 dim3 box_grid(const LensEpi2D &e, int nx, int ny) {
     int w = 0, h = 0;
@@ -861,6 +956,24 @@ extern "C" int lens_te2d_step_rows(const LensTE2D *g, const int *rowref, const L
 extern "C" int lens_tm2d_step_rows(const LensTM2D *g, const int *rowref, const LensStepTable *tab, const LensEpi2D *ep,
                                    int n0, int nsteps, void *stream) {
     return tm2d_run(g, tab, ep, nullptr, n0, nsteps, stream, rowref);
+}
+
+extern "C" int lens_te2d_row_table(const LensTE2D *g, const LensEpi2D *ep, int nsteps, int *rowref, void *stream) {
+    if (!rowref) return LENS_ERR_ARG;
+    if (!grid2d_ok(g) || !g->ce_e || !g->ce_h || !row_table_pays(g->nx, g->pitch, 5, nsteps) ||
+        (double)g->nx * g->ny < WIDE_TE || !wide_ok(ep ? *ep : empty_epi(), nullptr, {g->ez, g->hx, g->hy, g->ce_e, g->ce_h}))
+        return LENS_ERR_SIZE;
+    return row_table(RowArrays{{g->ce_e, g->ce_h}, {g->nx, g->nx}, 2}, g->nx, g->ny, g->pitch, rowref, stream);
+}
+
+extern "C" int lens_tm2d_row_table(const LensTM2D *g, const LensEpi2D *ep, int nsteps, int *rowref, void *stream) {
+    if (!rowref) return LENS_ERR_ARG;
+    if (!grid2d_ok(g) || !g->ca_x || !g->ca_y || (!g->da_x) != (!g->da_y) ||
+        !row_table_pays(g->nx, g->pitch, g->da_x ? 7 : 5, nsteps) || (double)g->nx * g->ny < WIDE_TM ||
+        !wide_ok(ep ? *ep : empty_epi(), nullptr, {g->ex, g->ey, g->hz, g->ca_x, g->ca_y, g->da_x, g->da_y}))
+        return LENS_ERR_SIZE;
+    return row_table(RowArrays{{g->ca_x, g->ca_y, g->da_x, g->da_y}, {g->nx - 1, g->nx, g->nx - 1, g->nx}, g->da_x ? 4 : 2},
+                     g->nx, g->ny, g->pitch, rowref, stream);
 }
 
 extern "C" int lens_te2d_step_driven(const LensTE2D *g, const LensStepTable *tab, const LensEpi2D *ep,

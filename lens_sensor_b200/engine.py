@@ -64,7 +64,8 @@ def strip_widths(c):
 
 def repeated_rows(arrays):
     """For every row of the (nx, pitch) arrays the first row of the run of equal rows it
-    lies in (equal bit for bit in all of them), int32 on the arrays' device."""
+    lies in (equal bit for bit in all of them), int32 on the arrays' device: the table of
+    lens_te2d_row_table / lens_tm2d_row_table in torch, its oracle."""
     nx = arrays[0].shape[0]
     new = torch.zeros(nx, dtype=torch.bool, device=arrays[0].device)
     new[0] = True
@@ -207,15 +208,8 @@ class Grid2D:
             ctypes.byref(self.s))
         self.rs_scratch = torch.empty(need, dtype=torch.uint8, device=dev) if need else None
         self.rs_err = torch.zeros(1, dtype=torch.int32, device=dev) if need else None
-        # coefficient rows that repeat, read once by the step by step passes of a grid beyond the chip,
-        # while the coefficients stay as they were given (the arrays' version counters tell)
-        self._coef = [a for a in ([self.ce_e, self.ce_h] if self.pol == 's' else
-                                  [self.ca_x, self.ca_y, self.da_x, self.da_y]) if a is not None]
-        self._coef_version = self._versions()
-        self.rowref = None if need or self._coef_version is None else repeated_rows(self._coef)
-
-    def _versions(self):
-        return None if any(a.is_inference() for a in self._coef) else [a._version for a in self._coef]
+        # row table of the wide passes (lens_te2d_row_table), formed anew by every step() that reads it
+        self.rowref = torch.empty(nx, dtype=torch.int32, device=dev) if not need else None
 
     # reference-shaped views of the resident fields
     def view(self, name):
@@ -252,13 +246,25 @@ class Grid2D:
         self.launches += 2 * max(0, int(nsteps))
         if drive is None:
             fn = self.lib.lens_te2d_step_rows if self.pol == 's' else self.lib.lens_tm2d_step_rows
-            rows = self.rowref if self.rowref is not None and self._versions() == self._coef_version else None
-            N.check(fn(ctypes.byref(self.s), _ptr(rows), ctypes.byref(table.s), e, int(n0), int(nsteps),
-                       _stream_ptr(stream)))
+            N.check(fn(ctypes.byref(self.s), self._row_table(e, nsteps, stream), ctypes.byref(table.s), e, int(n0),
+                       int(nsteps), _stream_ptr(stream)))
         else:
             fn = self.lib.lens_te2d_step_driven if self.pol == 's' else self.lib.lens_tm2d_step_driven
             N.check(fn(ctypes.byref(self.s), ctypes.byref(table.s), e, ctypes.byref(drive.s), int(n0),
                        int(nsteps), _stream_ptr(stream)))
+
+    def _row_table(self, e, nsteps, stream):
+        """The table of repeated coefficient rows for a span of nsteps, from the coefficients as
+        they are now (they may be written between calls in any way); NULL where the span would
+        not gain by it."""
+        if self.rowref is None:
+            return None
+        fn = self.lib.lens_te2d_row_table if self.pol == 's' else self.lib.lens_tm2d_row_table
+        st = fn(ctypes.byref(self.s), e, int(nsteps), _ptr(self.rowref), _stream_ptr(stream))
+        if st == N.ERR_SIZE:
+            return None
+        N.check(st)
+        return _ptr(self.rowref)
 
     def check(self):
         """Raise if a resident launch's wait between bands ran out (the fields hold NaN then)."""
