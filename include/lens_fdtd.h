@@ -234,7 +234,8 @@ typedef struct {
     int pec[4];
     LensSource src;              /* drives Ez (TE) or Ey (TM)                   */
     int dft_n0, dft_n1;          /* in the instance's own steps                 */
-    float *dft;                  /* (nx, pitch) x {re, im} or NULL              */
+    float *dft;                  /* (nx, pitch) x {re, im} or NULL; starts on 16
+                                    bytes (TE), 8 bytes (TM)                    */
     int n_start;                 /* batch step at which this instance's step 0
                                     runs: its own step is n - n_start (source
                                     time, DFT window, table row), so instances

@@ -551,6 +551,30 @@ __device__ __forceinline__ void e_tile(const LensInst2D *inst, const int *blk, c
     }
 }
 
+// Sums of four nodes: 16 bytes at a time where the array starts on 16 bytes (al; uniform over
+// an instance), else node by node (a TM instance's sums need the alignment of one node, 8 bytes).
+__device__ __forceinline__ void sums_in(float4 (&s)[2], const float *p, bool al) {
+    if (al) {
+        s[0] = reinterpret_cast<const float4 *>(p)[0];
+        s[1] = reinterpret_cast<const float4 *>(p)[1];
+    } else {
+        const float2 *q = reinterpret_cast<const float2 *>(p);
+        s[0] = make_float4(q[0].x, q[0].y, q[1].x, q[1].y);
+        s[1] = make_float4(q[2].x, q[2].y, q[3].x, q[3].y);
+    }
+}
+
+__device__ __forceinline__ void sums_out(float *p, const float4 (&s)[2], bool al) {
+    if (al) {
+        reinterpret_cast<float4 *>(p)[0] = s[0];
+        reinterpret_cast<float4 *>(p)[1] = s[1];
+    } else {
+        float2 *q = reinterpret_cast<float2 *>(p);
+        q[0] = make_float2(s[0].x, s[0].y); q[1] = make_float2(s[0].z, s[0].w);
+        q[2] = make_float2(s[1].x, s[1].y); q[3] = make_float2(s[1].z, s[1].w);
+    }
+}
+
 // TM node DFT of tile b: Ey averaged onto the nodes (fdtd2d_core.py:458-465), four
 // nodes of a row with one access to Ey and two to their sums (24 us a window step of
 // 16 instances, 6.9 M nodes, with an access per node and every node's own window test).
@@ -569,6 +593,7 @@ __device__ __forceinline__ void node_tile(const LensInst2D *inst, const int *blk
     const void *p1 = g.f(1);
     const int k = n - tab.t0;
     const float pr = __ldg(tab.pe + 2 * k), pim = __ldg(tab.pe + 2 * k + 1);
+    const bool al = (reinterpret_cast<uintptr_t>(dft) & 15) == 0;
     float ey[RB][VEC], left[RB];
     float4 s[RB][2];
 #pragma unroll
@@ -577,8 +602,7 @@ __device__ __forceinline__ void node_tile(const LensInst2D *inst, const int *blk
         const size_t o = (size_t)(i0 + r) * P + j0;
         f4_to(S::ld4(p1, o), ey[r]);
         left[r] = j0 > 0 ? S::ld(p1, o - 1) : 0.f;
-        s[r][0] = reinterpret_cast<const float4 *>(dft + 2 * o)[0];
-        s[r][1] = reinterpret_cast<const float4 *>(dft + 2 * o)[1];
+        sums_in(s[r], dft + 2 * o, al);
     }
 #pragma unroll
     for (int r = 0; r < RB; ++r) {
@@ -595,8 +619,7 @@ __device__ __forceinline__ void node_tile(const LensInst2D *inst, const int *blk
         s[r][0].z = __fmaf_rn(v[1], pr, s[r][0].z); s[r][0].w = __fmaf_rn(v[1], pim, s[r][0].w);
         s[r][1].x = __fmaf_rn(v[2], pr, s[r][1].x); s[r][1].y = __fmaf_rn(v[2], pim, s[r][1].y);
         s[r][1].z = __fmaf_rn(v[3], pr, s[r][1].z); s[r][1].w = __fmaf_rn(v[3], pim, s[r][1].w);
-        reinterpret_cast<float4 *>(dft + 2 * o)[0] = s[r][0];
-        reinterpret_cast<float4 *>(dft + 2 * o)[1] = s[r][1];
+        sums_out(dft + 2 * o, s[r], al);
     }
 }
 
