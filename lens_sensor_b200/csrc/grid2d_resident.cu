@@ -146,6 +146,13 @@ struct Plan {
     int nbands, ncol, nc;
 };
 
+// Let a kernel's launches ask for any dynamic shared memory the device has.  The limit
+// belongs to the kernel, whichever thread launches it: every call sets the same one, so no
+// call takes from another thread's plan what it was made with.
+bool rs_allow(const void *kernel, int smax) {
+    return cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, smax) == cudaSuccess;
+}
+
 // Band plan of a grid on this device: the row template and register split, the CTA count
 // and (when lo is not NULL) the first row of every band.  The bands minimise the largest
 // band cost, weighed by the CTAs that share an SM.  LENS_ERR_SIZE when the grid does not
@@ -187,7 +194,7 @@ int plan_(const LensInst2D &g, int nbox, Plan &p, short *lo) {
         const void *k = f.kernel(c.wide);
         const size_t sm = rs_smem(f, p.ncol, p.nc, nbox, false);
         int per = 0;
-        if (cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm) != cudaSuccess ||
+        if (!rs_allow(k, smax) ||
             cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, k, 32 * W, sm) != cudaSuccess)
             return LENS_ERR_CUDA;
         if (per < c.c) continue;
@@ -256,7 +263,6 @@ int run(const LensInst2D &g, const LensEpi2D *ep, const LensStepTable *tab, int 
         if (cudaGetDevice(&dev) == cudaSuccess &&
             cudaDeviceGetAttribute(&smax, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev) == cudaSuccess &&
             cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev) == cudaSuccess && smd <= (size_t)smax &&
-            cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smd) == cudaSuccess &&
             cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, kern, 32 * W, smd) == cudaSuccess &&
             (long)per * nsm >= p.nbands) {
             pl.hold = 1;
