@@ -807,8 +807,9 @@ int rs_plan_(const LensInst2D *inst, int ninst, int &rm, int &rows, int &W, int 
         const void *k = rs_kernel(cand, wide);
         const size_t sm = rs_smem(cand, W, nc);
         if (!k || sm > (size_t)smax) continue;
-        if (cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm) != cudaSuccess)
-            return LENS_ERR_CUDA;
+        // the limit belongs to the kernel, whichever thread launches it: every call sets the
+        // device's, so no call takes from another thread's plan what it was made with
+        if (cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, smax) != cudaSuccess) return LENS_ERR_CUDA;
         int per = 0;
         if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, k, 32 * W, sm) != cudaSuccess) return LENS_ERR_CUDA;
         const long avail = std::min((long)per * nsm, (long)RS_MAXCTA);

@@ -54,3 +54,38 @@ def test_grids_of_one_kernel(pols):
             assert torch.equal(getattr(g, q), getattr(b, q)), q
         if ea is not None:
             assert torch.equal(ea.dft, eb.dft)
+
+
+@pytest.mark.gpu
+def test_groups_of_one_kernel():
+    """Resident groups (lens_rs2d_run) of narrow TE and wide lossy TM instances, the same kernels at
+    other shared memory sizes."""
+    import torch
+    from dataclasses import replace
+    from lens_sensor_b200 import batch2d as B
+    from lens_sensor_b200 import engine as E
+    from lens_sensor_b200.workloads import sweep2d
+    dev = E._device(None)
+    specs = sweep2d(count=4)[0]
+    te, tm = (next(s for s in specs if s.pol == p) for p in 'sp')
+    sps = [replace(te, nx=160, ny=120), replace(tm, nx=160)]
+    steps, cut = 3000, 2
+    insts = [[B.Instance(sp, steps, torch.float32, dev, window=(10, steps)) for sp in sps] for _ in range(2)]
+    tabs = [E.StepTable(0, steps, q.spec.dt, q.omega, q.omega, E.cw_envelope(q.spec.f0)) for q in insts[0]]
+    groups = [B.ResidentGroup([q], dev) for q in insts[0]]
+
+    def job(g, tab):
+        def run(s):
+            for n in range(0, steps, cut):
+                g.step(tab, n, cut, s)
+        return run
+    errs = _together([job(g, t) for g, t in zip(groups, tabs)])
+    assert not errs, errs
+    for g, q, b, tab in zip(groups, *insts, tabs):
+        g.check()
+        one = B.ResidentGroup([b], dev)
+        one.step(tab, 0, steps)
+        torch.cuda.synchronize()
+        for x, y in zip(q.f, b.f):
+            assert torch.equal(x, y)
+        assert torch.equal(q.dft, b.dft)
