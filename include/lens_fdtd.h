@@ -194,8 +194,9 @@ int lens_tm2d_step_driven(const LensTM2D *g, const LensStepTable *tab, const Len
  * too little scratch) returns LENS_ERR_SIZE before anything is enqueued: step it with
  * the entries above.  The call zeroes scratch on `stream`.  Waits between bands are
  * bounded (seconds at most); if one runs out *err (a device int, zeroed once by the
- * caller) becomes nonzero, the launch ends and the band's fields become NaN.  The
- * launch takes every SM it plans for.                                         */
+ * caller) becomes nonzero, the launch ends, and in every band that left its step loop
+ * the fields, and whatever of the epilogue's sums its rows feed, become NaN.  The launch
+ * takes every SM it plans for.                                                */
 size_t lens_te2d_resident_bytes(const LensTE2D *g);
 size_t lens_tm2d_resident_bytes(const LensTM2D *g);
 int lens_te2d_resident(const LensTE2D *g, const LensStepTable *tab, const LensEpi2D *ep, int n0, int nsteps,
@@ -208,6 +209,8 @@ int lens_tm2d_resident(const LensTM2D *g, const LensStepTable *tab, const LensEp
  * nonzero, every band leaves its step loop.  Needs two bands and nsteps >= 3.   */
 int lens_te2d_resident_watchdog_test(const LensTE2D *g, const LensStepTable *tab, int n0, int nsteps, void *scratch,
                                      size_t bytes, int *err, void *stream);
+int lens_tm2d_resident_watchdog_test(const LensTM2D *g, const LensStepTable *tab, const LensEpi2D *ep, int n0, int nsteps,
+                                     void *scratch, size_t bytes, int *err, void *stream);
 
 /* ------------------------------------------------------- batched 2D solves
  * Many independent 2D solves of uneven sizes (TE and TM mixed) advanced together:

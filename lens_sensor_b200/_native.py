@@ -176,6 +176,8 @@ SIGNATURES = {
                                    ctypes.c_size_t, c_void_p, c_void_p]),
     'lens_te2d_resident_watchdog_test': (c_int, [POINTER(TE2D), POINTER(StepTable), c_int, c_int, c_void_p,
                                                  ctypes.c_size_t, c_void_p, c_void_p]),
+    'lens_tm2d_resident_watchdog_test': (c_int, [POINTER(TM2D), POINTER(StepTable), POINTER(Epi2D), c_int, c_int, c_void_p,
+                                                 ctypes.c_size_t, c_void_p, c_void_p]),
     'lens_version': (c_int, []),
     'lens_status_string': (ctypes.c_char_p, [c_int]),
     'lens_abi_sizes': (c_int, [POINTER(c_int), c_int]),

@@ -306,3 +306,8 @@ extern "C" int lens_te2d_resident_watchdog_test(const LensTE2D *g, const LensSte
                                                 void *scratch, size_t bytes, int *err, void *stream) {
     return g ? run(inst_of(*g), nullptr, tab, n0, nsteps, scratch, bytes, err, stream, 1024, 1) : LENS_ERR_ARG;
 }
+
+extern "C" int lens_tm2d_resident_watchdog_test(const LensTM2D *g, const LensStepTable *tab, const LensEpi2D *ep, int n0,
+                                                int nsteps, void *scratch, size_t bytes, int *err, void *stream) {
+    return g ? run(inst_of(*g), ep, tab, n0, nsteps, scratch, bytes, err, stream, 1024, 1) : LENS_ERR_ARG;
+}

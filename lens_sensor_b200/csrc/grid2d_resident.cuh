@@ -21,8 +21,8 @@
 // thread of the same columns polls them at the end of its next H phase until the
 // tag of the step it needs appears, so that the hop passes under the rest of both
 // phases.  Every poll is bounded; a wait that runs out sets *err, and all CTAs
-// leave the step loop at their next CTA barrier (or when they see *err), write
-// their state back and end.  Each slot of the halo rows is double-buffered by step
+// leave the step loop at their next CTA barrier (or when they see *err), turn their
+// rows of the fields and sums into NaN, write them back and end.  Each slot of the halo rows is double-buffered by step
 // parity; a band publishes step n+1 only after it has read both neighbours' step n,
 // which they published after reading its step n-1, the slot's last content.
 //
@@ -883,7 +883,10 @@ __device__ __forceinline__ bool rs_loop(Th<RM> &t, const Band &B, const GPlan &p
             if (POL == 0) edge_out<RM, true>(xb, w, t.b, f2(0.f));
             else edge_out<RM, true>(xb, w, t.c, t.gc);
         }
-        if (__syncthreads_or(bad)) break;
+        if (__syncthreads_or(bad)) {  // one thread's wait ran out: the whole band's results are invalid
+            bad = true;
+            break;
+        }
 
         // ------------------------------------------------------------ E phase
         float x[EP];
@@ -1077,14 +1080,34 @@ __device__ __forceinline__ void rs_band(const GPlan &pl, const LensStepTable &ta
     else if (form == 0u) bad = rs_loop<RM, POL, 0u>(t, B, pl, tab, n0, nsteps, halo, err, prev, next, box, zb, hold, sdft, bacc);
     else if (form == V_N) bad = rs_loop<RM, POL, V_N>(t, B, pl, tab, n0, nsteps, halo, err, prev, next, box, zb, hold, sdft, bacc);
     else bad = rs_loop<RM, POL, V_N | V_Y>(t, B, pl, tab, n0, nsteps, halo, err, prev, next, box, zb, hold, sdft, bacc);
-    if (bad) {  // the results are invalid: make that plain in the fields too
+    const LensEpi2D &ep = pl.ep;
+    if (bad) {  // the results are invalid: make that plain in the fields and in every sum of the band
+        const float nan = __int_as_float(0x7fc00000);
         atomicOr(err, 1);
 #pragma unroll
-        for (int r = 0; r < RM; ++r) t.a[r] = t.b[r] = t.c[r] = f2(__int_as_float(0x7fc00000));
+        for (int r = 0; r < RM; ++r) {  // the components' own cells: what lies beyond them stays as it is
+            const unsigned h = B.lo + r < B.nx - 1 ? ~0u : 0u, e = POL == 0 ? ~0u : h;
+            t.a[r] = bsel2(t.lt0 & e, t.lt1 & e, f2(nan), t.a[r]);
+            t.b[r] = bsel2(t.hx0, t.hx1, f2(nan), t.b[r]);
+            t.c[r] = bsel2(h & (POL == 0 ? t.lt0 : t.hx0), h & (POL == 0 ? t.lt1 : t.hx1), f2(nan), t.c[r]);
+        }
+        for (int b = 0; b < ep.nbox && box; ++b) bacc[b * 32 * W] = nan;
+        for (int r = 0; r < R; ++r)
+            for (int c = 0; c < 2; ++c) {
+                if (!lt[c]) continue;
+                const size_t o = (size_t)(B.lo + r) * B.P + j + c;
+                float *const sum[3] = {ep.dft, ep.dft_ex, ep.dft_prev};
+                for (int q = 0; q < 3; ++q)
+                    if (sum[q]) reinterpret_cast<float4 *>(sum[q])[o] = make_float4(nan, nan, nan, nan);
+                if (ep.iavg) ep.iavg[o] = nan;
+                for (int p = 0; p < ep.nplane; ++p)
+                    for (int q = 0; q < 4; ++q)
+                        if (ep.plane[p] == B.lo + r) ep.plane_acc[((size_t)p * 4 + q) * B.P + j + c] = nan;
+            }
     }
 
     // ---- state out
-    if (hold && lt[0])
+    if (hold && !bad && lt[0])
         for (int r = 0; r < R; ++r) {
             const float4 *l = reinterpret_cast<const float4 *>(sdft) + (size_t)r * NS;
             gdft[(size_t)r * B.P] = l[0];

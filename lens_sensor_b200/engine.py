@@ -267,7 +267,7 @@ class Grid2D:
         return _ptr(self.rowref)
 
     def check(self):
-        """Raise if a resident launch's wait between bands ran out (the fields hold NaN then)."""
+        """Raise if a resident launch's wait between bands ran out (fields and sums hold NaN then)."""
         if self.rs_err is not None and int(self.rs_err.item()) != 0:
             raise N.LensError('resident 2D launch: a wait between bands timed out (results invalid)')
 
