@@ -438,6 +438,7 @@ def run_beads_stitched(wg_mat, bead_mat, bead_d_um, dx_nm, save_frames, n_snapsh
         drive = (E.Drive2D(grid, hand, wtap, env_t, ph_t.real, ph_t.imag)
                  if (w > 0 and hand is not None) else None)
         grid.step(tab, 0, steps_win, ep, drive=drive)
+        _check(grid)
         a = ep.phasor('dft_raw' if pol == 'p' else 'dft', kind='stitch')
         s_ = sc.to(a.device)
         Ew_d = torch.complex(a.real.float() * s_, a.imag.float() * s_)
