@@ -208,6 +208,7 @@ class Grid2D:
             ctypes.byref(self.s))
         self.rs_scratch = torch.empty(need, dtype=torch.uint8, device=dev) if need else None
         self.rs_err = torch.zeros(1, dtype=torch.int32, device=dev) if need else None
+        self.rs_stream = None       # stream of the last resident launch
         # row table of the wide passes (lens_te2d_row_table), formed anew by every step() that reads it
         self.rowref = torch.empty(nx, dtype=torch.int32, device=dev) if not need else None
 
@@ -242,6 +243,7 @@ class Grid2D:
                     self.rs_scratch.numel(), _ptr(self.rs_err), _stream_ptr(stream))
             if st != N.ERR_SIZE:      # else: a call that only the steps below carry
                 self.launches += 1
+                self.rs_stream = stream if stream is not None else torch.cuda.current_stream()
                 return N.check(st)
         self.launches += 2 * max(0, int(nsteps))
         if drive is None:
@@ -267,7 +269,10 @@ class Grid2D:
         return _ptr(self.rowref)
 
     def check(self):
-        """Raise if a resident launch's wait between bands ran out (fields and sums hold NaN then)."""
+        """Wait for the last resident launch; raise if a wait between its bands ran out (fields and
+        sums hold NaN then)."""
+        if self.rs_stream is not None:      # it may lie on another stream than this one
+            self.rs_stream.synchronize()
         if self.rs_err is not None and int(self.rs_err.item()) != 0:
             raise N.LensError('resident 2D launch: a wait between bands timed out (results invalid)')
 

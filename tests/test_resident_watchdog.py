@@ -41,3 +41,20 @@ def test_whole_bands_and_their_sums_are_nan(hold):
         full = getattr(g, q).clone()
         full[:g.view(q).shape[0], :g.view(q).shape[1]] = 0
         assert not bool(full.any()), q
+
+
+@pytest.mark.gpu
+def test_check_waits_for_the_launch():
+    """The error word of a launch on another stream is read after that launch."""
+    import torch
+    from lens_sensor_b200 import engine as E
+    g = _grid('s', 140, 96, False, 5)
+    tab = E.StepTable(7, 20, g.dt, 2.2e15, 2.2e15, E.cw_envelope(3.5e14))
+    torch.cuda.synchronize()
+    s = torch.cuda.Stream()
+    with torch.cuda.stream(s):
+        torch.cuda._sleep(400_000_000)      # 0.2 s
+        g.rs_err.fill_(1)                   # as a wait that ran out leaves it
+    g.step(tab, 7, 20, stream=s)
+    with pytest.raises(N.LensError):
+        g.check()
