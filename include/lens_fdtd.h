@@ -189,14 +189,14 @@ int lens_tm2d_step_driven(const LensTM2D *g, const LensStepTable *tab, const Len
  * more per SM): bands of x rows exchange one row per step through L2.  Fields, psi and
  * sums hold the bits that lens_te2d_step / lens_tm2d_step would leave (FP64 sums of boxes
  * and planes to their last digits), so a caller may mix the two.  *_bytes: device scratch
- * the launch needs, 0 when the grid does not fit.  A call that the resident launch does
- * not carry (the epilogue's dft_raw, ex2 or nsx planes, a capturing stream, nsteps < 1,
- * too little scratch) returns LENS_ERR_SIZE before anything is enqueued: step it with
- * the entries above.  The call zeroes scratch on `stream`.  Waits between bands are
- * bounded (seconds at most); if one runs out *err (a device int, zeroed once by the
- * caller) becomes nonzero, the launch ends, and in every band that left its step loop
- * the fields, and whatever of the epilogue's sums its rows feed, become NaN.  The launch
- * takes every SM it plans for.                                                */
+ * that is enough for every epilogue the grid fits with, 0 when it fits with none.  A call
+ * that the resident launch does not carry (the epilogue's dft_raw, ex2 or nsx planes, more
+ * boxes than fit, a capturing stream, nsteps < 1, too little scratch) returns LENS_ERR_SIZE
+ * before anything is enqueued: step it with the entries above.  The call zeroes scratch on
+ * `stream`.  Waits between bands are bounded (seconds at most); if one runs out *err (a
+ * device int, zeroed once by the caller) becomes nonzero, the launch ends, and in every
+ * band that left its step loop the fields, and whatever of the epilogue's sums its rows
+ * feed, become NaN.  The launch takes every SM it plans for.                  */
 size_t lens_te2d_resident_bytes(const LensTE2D *g);
 size_t lens_tm2d_resident_bytes(const LensTM2D *g);
 int lens_te2d_resident(const LensTE2D *g, const LensStepTable *tab, const LensEpi2D *ep, int n0, int nsteps,

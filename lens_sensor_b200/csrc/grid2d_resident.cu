@@ -219,6 +219,17 @@ int plan(const LensInst2D &g, int nbox, Plan &p, short *lo) {
 
 size_t scratch_bytes(const Plan &p) { return (size_t)p.nbands * 4 * ((p.ncol + 63) / 64 * 64) * sizeof(unsigned long long); }
 
+// The most scratch a call may need.  A call's plan depends on its boxes, whose sums take
+// shared memory: with fewer of them more CTAs may share an SM, with more and shorter bands.
+size_t most_scratch(const LensInst2D &g) {
+    size_t most = 0;
+    for (int nbox = 0; nbox <= LENS_MAX_BOX; ++nbox) {
+        Plan p{};
+        if (plan(g, nbox, p, nullptr) == LENS_OK) most = std::max(most, scratch_bytes(p));
+    }
+    return most;
+}
+
 int run(const LensInst2D &g, const LensEpi2D *ep, const LensStepTable *tab, int n0, int nsteps, void *scratch, size_t bytes,
         int *err, void *stream, unsigned tries, int wd) {
     if (!scratch || !err || nsteps < 1 || !lens_table_ok(tab, n0, nsteps)) return LENS_ERR_SIZE;
@@ -282,15 +293,9 @@ int run(const LensInst2D &g, const LensEpi2D *ep, const LensStepTable *tab, int 
 
 }  // namespace
 
-extern "C" size_t lens_te2d_resident_bytes(const LensTE2D *g) {
-    Plan p{};
-    return g && plan(inst_of(*g), LENS_MAX_BOX, p, nullptr) == LENS_OK ? scratch_bytes(p) : 0;
-}
+extern "C" size_t lens_te2d_resident_bytes(const LensTE2D *g) { return g ? most_scratch(inst_of(*g)) : 0; }
 
-extern "C" size_t lens_tm2d_resident_bytes(const LensTM2D *g) {
-    Plan p{};
-    return g && plan(inst_of(*g), LENS_MAX_BOX, p, nullptr) == LENS_OK ? scratch_bytes(p) : 0;
-}
+extern "C" size_t lens_tm2d_resident_bytes(const LensTM2D *g) { return g ? most_scratch(inst_of(*g)) : 0; }
 
 extern "C" int lens_te2d_resident(const LensTE2D *g, const LensStepTable *tab, const LensEpi2D *ep, int n0, int nsteps,
                                   void *scratch, size_t bytes, int *err, void *stream) {
