@@ -204,6 +204,12 @@ int lens_te2d_resident(const LensTE2D *g, const LensStepTable *tab, const LensEp
 int lens_tm2d_resident(const LensTM2D *g, const LensStepTable *tab, const LensEpi2D *ep, int n0, int nsteps,
                        void *scratch, size_t bytes, int *err, void *stream);
 
+/* The plan of that launch for nbox detector boxes: *bands, *rows, the most rows of a
+ * band, and *threads, 256 or 384, the register split (the threads a CTA may have).
+ * LENS_ERR_SIZE when the grid does not fit.                                   */
+int lens_te2d_resident_rows(const LensTE2D *g, int nbox, int *rows, int *threads, int *bands);
+int lens_tm2d_resident_rows(const LensTM2D *g, int nbox, int *rows, int *threads, int *bands);
+
 /* Watchdog self-test (no counterpart in the reference): the launch with every wait cut
  * to 1024 polls and the second band withholding its first E row of step 1; *err becomes
  * nonzero, every band leaves its step loop.  Needs two bands and nsteps >= 3.   */

@@ -170,6 +170,8 @@ SIGNATURES = {
                                         c_void_p, ctypes.c_size_t, c_void_p, c_void_p]),
     'lens_te2d_resident_bytes': (ctypes.c_size_t, [POINTER(TE2D)]),
     'lens_tm2d_resident_bytes': (ctypes.c_size_t, [POINTER(TM2D)]),
+    'lens_te2d_resident_rows': (c_int, [POINTER(TE2D), c_int] + [POINTER(c_int)] * 3),
+    'lens_tm2d_resident_rows': (c_int, [POINTER(TM2D), c_int] + [POINTER(c_int)] * 3),
     'lens_te2d_resident': (c_int, [POINTER(TE2D), POINTER(StepTable), POINTER(Epi2D), c_int, c_int, c_void_p,
                                    ctypes.c_size_t, c_void_p, c_void_p]),
     'lens_tm2d_resident': (c_int, [POINTER(TM2D), POINTER(StepTable), POINTER(Epi2D), c_int, c_int, c_void_p,

@@ -230,6 +230,17 @@ size_t most_scratch(const LensInst2D &g) {
     return most;
 }
 
+int rows_of(const LensInst2D &g, int nbox, int *rows, int *threads, int *bands) {
+    if (nbox < 0 || nbox > LENS_MAX_BOX || !rows || !threads || !bands) return LENS_ERR_ARG;
+    Plan p{};
+    const int st = plan(g, nbox, p, nullptr);
+    if (st != LENS_OK) return st;
+    *rows = p.form->rm;
+    *threads = p.wide ? 384 : 256;
+    *bands = p.nbands;
+    return LENS_OK;
+}
+
 int run(const LensInst2D &g, const LensEpi2D *ep, const LensStepTable *tab, int n0, int nsteps, void *scratch, size_t bytes,
         int *err, void *stream, unsigned tries, int wd) {
     if (!scratch || !err || nsteps < 1 || !lens_table_ok(tab, n0, nsteps)) return LENS_ERR_SIZE;
@@ -292,6 +303,14 @@ int run(const LensInst2D &g, const LensEpi2D *ep, const LensStepTable *tab, int 
 }
 
 }  // namespace
+
+extern "C" int lens_te2d_resident_rows(const LensTE2D *g, int nbox, int *rows, int *threads, int *bands) {
+    return g ? rows_of(inst_of(*g), nbox, rows, threads, bands) : LENS_ERR_ARG;
+}
+
+extern "C" int lens_tm2d_resident_rows(const LensTM2D *g, int nbox, int *rows, int *threads, int *bands) {
+    return g ? rows_of(inst_of(*g), nbox, rows, threads, bands) : LENS_ERR_ARG;
+}
 
 extern "C" size_t lens_te2d_resident_bytes(const LensTE2D *g) { return g ? most_scratch(inst_of(*g)) : 0; }
 

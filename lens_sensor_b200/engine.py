@@ -83,6 +83,45 @@ def repeated_rows(arrays):
 # 83.3 (at 1 step 61 / 29, at 16 steps 156 / 306).
 RS_MIN_STEPS = 4
 
+# The same for bands whose rows and sums do not fit the registers: from 10 rows where a thread
+# has 168 (a CTA of more than 8 warps, or several on an SM), from 16 where it has 255.  Every
+# sum a step then costs more in the resident launch than in the passes.  By the sums a step runs
+# (DFT, TM Ex, comparison window, average), TE and TM; us a call, resident / step by step, on
+# either side of a line: TE 2400 x 513 with 3 sums 467 / 445 at 12 steps and 852 / 880 at 24, TE
+# 7000 x 90 with 2 275 / 254 and 471 / 506 at the same, TM 2100 x 513 with 4 612 / 599 at 12 and
+# 1117 / 1190 at 24, TE 5000 x 180 with 1 113 / 99 at 4 and 120 / 121 at 5, TM 2400 x 448 with 4
+# 235 / 189 at 4 and 607 / 731 at 16; the TM forms marked NEVER lose at any length: 2400 x 513
+# with 4 sums 4098 / 3723 at 64 steps, 7000 x 90 with 3 1930 / 1847.
+NEVER = 1 << 30
+RS_SPILL_STEPS = [  # crowded (168 registers or several CTAs an SM), least rows, steps TE, steps TM
+    (True, 18, (5, 6, 12, 20), (6, 7, 32, 32, NEVER)),
+    (True, 16, (4, 6, 10, 12), (5, 5, 10, 12, 20)),
+    (True, 10, (4, 5, 7, 8), (4, 4, 5, 6, 6)),
+    (False, 20, (5, 6, 10, 14), (5, 4, 7, 9, 11)),
+    (False, 16, (4, 5, 6, 10), (4, 4, 5, 6, 7))]
+
+
+def resident_steps(pol, rows, threads, bands, sums):
+    """Steps from which a span that runs `sums` sums a step is faster on the resident launch of
+    this plan (lens_te2d_resident_rows) than step by step."""
+    crowded = threads == 384 or bands > 148
+    for crowd, least, te, tm in RS_SPILL_STEPS:
+        if crowd == crowded and rows >= least:
+            t = te if pol == 's' else tm
+            n = t[min(sums, len(t) - 1)]
+            return NEVER if pol == 'p' and sums == 3 and rows >= 18 and crowded and threads == 256 else n
+    return 0
+
+
+def sums_a_step(e, n0, nsteps):
+    """Sums of an epilogue (_native.Epi2D) that a step of [n0, n0 + nsteps) runs, on average."""
+    def met(a, b):
+        return max(0, min(b, n0 + nsteps) - max(a, n0))
+    w = met(e.dft_n0, e.dft_n1)
+    k = (w if e.dft else 0) + (w if e.dft_ex else 0) + (met(e.prev_n0, e.prev_n1) if e.dft_prev else 0) + \
+        (met(e.iavg_n0, n0 + nsteps) if e.iavg else 0)
+    return (2 * k + nsteps) // (2 * nsteps)
+
 
 class _Axis:
     """Device copy of one CPML axis (b, c, 1/kappa on integer and half nodes).
@@ -209,6 +248,12 @@ class Grid2D:
         self.rs_scratch = torch.empty(need, dtype=torch.uint8, device=dev) if need else None
         self.rs_err = torch.zeros(1, dtype=torch.int32, device=dev) if need else None
         self.rs_stream = None       # stream of the last resident launch
+        self.rs_plan = None         # rows, threads and bands of that launch
+        if need:
+            plan = [ctypes.c_int() for _ in range(3)]
+            fn = self.lib.lens_te2d_resident_rows if self.pol == 's' else self.lib.lens_tm2d_resident_rows
+            N.check(fn(ctypes.byref(self.s), 0, *map(ctypes.byref, plan)))
+            self.rs_plan = tuple(v.value for v in plan)
         # row table of the wide passes (lens_te2d_row_table), formed anew by every step() that reads it
         self.rowref = torch.empty(nx, dtype=torch.int32, device=dev) if not need else None
 
@@ -237,7 +282,8 @@ class Grid2D:
 
     def step(self, table, n0, nsteps, epi=None, stream=None, drive=None):
         e = ctypes.byref(epi.s) if epi is not None else None
-        if drive is None and self.rs_scratch is not None and nsteps >= RS_MIN_STEPS:
+        if drive is None and self.rs_scratch is not None and nsteps >= RS_MIN_STEPS and \
+                nsteps >= resident_steps(self.pol, *self.rs_plan, sums_a_step(epi.s, int(n0), int(nsteps)) if epi else 0):
             fn = self.lib.lens_te2d_resident if self.pol == 's' else self.lib.lens_tm2d_resident
             st = fn(ctypes.byref(self.s), ctypes.byref(table.s), e, int(n0), int(nsteps), _ptr(self.rs_scratch),
                     self.rs_scratch.numel(), _ptr(self.rs_err), _stream_ptr(stream))
