@@ -95,7 +95,7 @@ RS_MIN_STEPS = 4
 NEVER = 1 << 30
 RS_SPILL_STEPS = [  # crowded (168 registers or several CTAs an SM), least rows, steps TE, steps TM
     (True, 18, (5, 6, 12, 20), (6, 7, 32, 32, NEVER)),
-    (True, 16, (4, 6, 10, 12), (5, 5, 10, 12, 20)),
+    (True, 16, (5, 6, 10, 12), (5, 5, 10, 12, 20)),
     (True, 10, (4, 5, 7, 8), (4, 4, 5, 6, 6)),
     (False, 20, (5, 6, 10, 14), (5, 4, 7, 9, 11)),
     (False, 16, (4, 5, 6, 10), (4, 4, 5, 6, 7))]
@@ -105,6 +105,8 @@ def resident_steps(pol, rows, threads, bands, sums):
     """Steps from which a span that runs `sums` sums a step is faster on the resident launch of
     this plan (lens_te2d_resident_rows) than step by step."""
     crowded = threads == 384 or bands > 148
+    if crowded and threads == 256 and rows == 14:   # narrow and long: 6000 x 60 takes as many as 6500 x 120
+        rows = 16
     for crowd, least, te, tm in RS_SPILL_STEPS:
         if crowd == crowded and rows >= least:
             t = te if pol == 's' else tm
