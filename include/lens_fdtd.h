@@ -184,6 +184,13 @@ int lens_te2d_step_driven(const LensTE2D *g, const LensStepTable *tab, const Len
 int lens_tm2d_step_driven(const LensTM2D *g, const LensStepTable *tab, const LensEpi2D *ep,
                           const LensDrive2D *drive, int n0, int nsteps, void *stream);
 
+/* Kernel launches that lens_*_step, lens_*_step_rows (drive NULL) or lens_*_step_driven
+ * makes for a span, or < 0 where the call is refused.  Nothing is launched.   */
+int lens_te2d_step_launches(const LensTE2D *g, const LensStepTable *tab, const LensEpi2D *ep, const LensDrive2D *drive,
+                            int n0, int nsteps);
+int lens_tm2d_step_launches(const LensTM2D *g, const LensStepTable *tab, const LensEpi2D *ep, const LensDrive2D *drive,
+                            int n0, int nsteps);
+
 /* The same steps in ONE cooperative launch that keeps the fields in registers, for a
  * grid whose state fits on the chip (ny <= 768, at most 20 rows per band and one band or
  * more per SM): bands of x rows exchange one row per step through L2.  Fields, psi and

@@ -877,39 +877,50 @@ dim3 box_grid(const LensEpi2D &e, int nx, int ny) {
     return w > 0 && h > 0 ? dim3((w + BX - 1) / BX, (h + BY * BOXR - 1) / (BY * BOXR), e.nbox) : dim3(0, 1, 1);
 }
 
+// The launches of a span, made or (count) only counted.
+struct Launch {
+    int *count;
+    template <class F>
+    void operator()(F launch) const {
+        if (count) ++*count;
+        else launch();
+    }
+};
+
 int te2d_run(const LensTE2D *g, const LensStepTable *tab, const LensEpi2D *ep, const LensDrive2D *dr, int n0,
-             int nsteps, void *stream, const int *rowref = nullptr) {
+             int nsteps, void *stream, const int *rowref = nullptr, int *count = nullptr) {
     if (!grid2d_ok(g) || !psi2d_ok(g) || !g->ez || !g->hx || !g->hy || !g->ce_e || !g->ce_h || nsteps < 0 ||
         !lens_table_ok(tab, n0, nsteps) || !epi2d_ok(ep, tab, g->nx) || !drive2d_ok(dr, tab, g->nx))
         return LENS_ERR_ARG;
     const LensEpi2D e = ep ? *ep : empty_epi();
     const LensDrive2D d = dr ? *dr : LensDrive2D{};
     cudaStream_t s = static_cast<cudaStream_t>(stream);
+    const Launch go{count};
     const dim3 blk(BX, BY), grd((g->ny + BX - 1) / BX, (g->nx + BY - 1) / BY);
     const double cells = (double)g->nx * g->ny;
     if (cells >= WIDE_TE && wide_ok(e, dr, {g->ez, g->hx, g->hy, g->ce_e, g->ce_h})) {
         const dim3 wb(BX, WT), wg((g->ny + BX * WV - 1) / (BX * WV), (g->nx + WT * WR - 1) / (WT * WR)), bg = box_grid(e, g->nx, g->ny);
         for (int n = n0; n < n0 + nsteps; ++n) {
-            te2d_h_wide<<<wg, wb, 0, s>>>(*g);
+            go([&] { te2d_h_wide<<<wg, wb, 0, s>>>(*g); });
             if (cells < WIDE_TE_WINDOW && epi2d_beyond_boxes(&e, n)) {
-                te2d_e<<<grd, blk, 0, s>>>(*g, *tab, e, n, d);
+                go([&] { te2d_e<<<grd, blk, 0, s>>>(*g, *tab, e, n, d); });
                 continue;
             }
-            te2d_e_wide<<<wg, wb, 0, s>>>(*g, rowref, *tab, n);
-            if (epi2d_beyond_boxes(&e, n)) te2d_epi<<<grd, blk, 0, s>>>(*g, *tab, e, n);
-            else if (bg.x > 0) box2d<<<bg, blk, 0, s>>>(*g, e);
+            go([&] { te2d_e_wide<<<wg, wb, 0, s>>>(*g, rowref, *tab, n); });
+            if (epi2d_beyond_boxes(&e, n)) go([&] { te2d_epi<<<grd, blk, 0, s>>>(*g, *tab, e, n); });
+            else if (bg.x > 0) go([&] { box2d<<<bg, blk, 0, s>>>(*g, e); });
         }
-        return lens_cuda_status();
+        return count ? LENS_OK : lens_cuda_status();
     }
     for (int n = n0; n < n0 + nsteps; ++n) {
-        te2d_h<<<grd, blk, 0, s>>>(*g);
-        te2d_e<<<grd, blk, 0, s>>>(*g, *tab, e, n, d);
+        go([&] { te2d_h<<<grd, blk, 0, s>>>(*g); });
+        go([&] { te2d_e<<<grd, blk, 0, s>>>(*g, *tab, e, n, d); });
     }
-    return lens_cuda_status();
+    return count ? LENS_OK : lens_cuda_status();
 }
 
 int tm2d_run(const LensTM2D *g, const LensStepTable *tab, const LensEpi2D *ep, const LensDrive2D *dr, int n0,
-             int nsteps, void *stream, const int *rowref = nullptr) {
+             int nsteps, void *stream, const int *rowref = nullptr, int *count = nullptr) {
     if (!grid2d_ok(g) || !psi2d_ok(g) || !g->ex || !g->ey || !g->hz || !g->ca_x || !g->ca_y ||
         (!g->da_x) != (!g->da_y) || nsteps < 0 || !lens_table_ok(tab, n0, nsteps) ||
         !epi2d_ok(ep, tab, g->nx) || !drive2d_ok(dr, tab, g->nx))
@@ -917,23 +928,24 @@ int tm2d_run(const LensTM2D *g, const LensStepTable *tab, const LensEpi2D *ep, c
     const LensEpi2D e = ep ? *ep : empty_epi();
     const LensDrive2D d = dr ? *dr : LensDrive2D{};
     cudaStream_t s = static_cast<cudaStream_t>(stream);
+    const Launch go{count};
     const dim3 blk(BX, BY), grd((g->ny + BX - 1) / BX, (g->nx + BY - 1) / BY);
     if ((double)g->nx * g->ny >= WIDE_TM && wide_ok(e, dr, {g->ex, g->ey, g->hz, g->ca_x, g->ca_y, g->da_x, g->da_y})) {
         const dim3 wb(BX, WT), wg((g->ny + BX * WV - 1) / (BX * WV), (g->nx + WT * WR - 1) / (WT * WR)), bg = box_grid(e, g->nx, g->ny);
         for (int n = n0; n < n0 + nsteps; ++n) {
-            tm2d_h_wide<<<wg, wb, 0, s>>>(*g);
-            tm2d_e_wide<<<wg, wb, 0, s>>>(*g, rowref, *tab, n);
-            if (epi2d_beyond_boxes(&e, n)) tm2d_epi<<<grd, blk, 0, s>>>(*g, *tab, e, n);
-            else if (bg.x > 0) box2d<<<bg, blk, 0, s>>>(*g, e);
+            go([&] { tm2d_h_wide<<<wg, wb, 0, s>>>(*g); });
+            go([&] { tm2d_e_wide<<<wg, wb, 0, s>>>(*g, rowref, *tab, n); });
+            if (epi2d_beyond_boxes(&e, n)) go([&] { tm2d_epi<<<grd, blk, 0, s>>>(*g, *tab, e, n); });
+            else if (bg.x > 0) go([&] { box2d<<<bg, blk, 0, s>>>(*g, e); });
         }
-        return lens_cuda_status();
+        return count ? LENS_OK : lens_cuda_status();
     }
     for (int n = n0; n < n0 + nsteps; ++n) {
-        tm2d_h<<<grd, blk, 0, s>>>(*g);
-        tm2d_e<<<grd, blk, 0, s>>>(*g, *tab, n, d);
-        if (epi2d_active(&e, n)) tm2d_epi<<<grd, blk, 0, s>>>(*g, *tab, e, n);
+        go([&] { tm2d_h<<<grd, blk, 0, s>>>(*g); });
+        go([&] { tm2d_e<<<grd, blk, 0, s>>>(*g, *tab, n, d); });
+        if (epi2d_active(&e, n)) go([&] { tm2d_epi<<<grd, blk, 0, s>>>(*g, *tab, e, n); });
     }
-    return lens_cuda_status();
+    return count ? LENS_OK : lens_cuda_status();
 }
 
 }  // namespace
@@ -956,6 +968,20 @@ extern "C" int lens_te2d_step_rows(const LensTE2D *g, const int *rowref, const L
 extern "C" int lens_tm2d_step_rows(const LensTM2D *g, const int *rowref, const LensStepTable *tab, const LensEpi2D *ep,
                                    int n0, int nsteps, void *stream) {
     return tm2d_run(g, tab, ep, nullptr, n0, nsteps, stream, rowref);
+}
+
+extern "C" int lens_te2d_step_launches(const LensTE2D *g, const LensStepTable *tab, const LensEpi2D *ep,
+                                       const LensDrive2D *drive, int n0, int nsteps) {
+    int n = 0;
+    const int st = te2d_run(g, tab, ep, drive, n0, nsteps, nullptr, nullptr, &n);
+    return st == LENS_OK ? n : st;
+}
+
+extern "C" int lens_tm2d_step_launches(const LensTM2D *g, const LensStepTable *tab, const LensEpi2D *ep,
+                                       const LensDrive2D *drive, int n0, int nsteps) {
+    int n = 0;
+    const int st = tm2d_run(g, tab, ep, drive, n0, nsteps, nullptr, nullptr, &n);
+    return st == LENS_OK ? n : st;
 }
 
 extern "C" int lens_te2d_row_table(const LensTE2D *g, const LensEpi2D *ep, int nsteps, int *rowref, void *stream) {

@@ -243,7 +243,7 @@ class Grid2D:
                             _ptr(self.psi['eyx']), pec4, s)
 
         # scratch and error word of the resident launch (lens_te2d_resident), when the grid fits the chip;
-        # launches step() has made (a resident launch once per call, the passes H and E once per step)
+        # launches: kernel launches step() has made
         self.launches = 0
         need = (self.lib.lens_te2d_resident_bytes if self.pol == 's' else self.lib.lens_tm2d_resident_bytes)(
             ctypes.byref(self.s))
@@ -293,15 +293,21 @@ class Grid2D:
                 self.launches += 1
                 self.rs_stream = stream if stream is not None else torch.cuda.current_stream()
                 return N.check(st)
-        self.launches += 2 * max(0, int(nsteps))
+        te = self.pol == 's'
+        d = ctypes.byref(drive.s) if drive is not None else None
+        span = (ctypes.byref(table.s), e)
+        fn = self.lib.lens_te2d_step_launches if te else self.lib.lens_tm2d_step_launches
+        made = fn(ctypes.byref(self.s), *span, d, int(n0), int(nsteps))
+        N.check(min(0, made))
         if drive is None:
-            fn = self.lib.lens_te2d_step_rows if self.pol == 's' else self.lib.lens_tm2d_step_rows
-            N.check(fn(ctypes.byref(self.s), self._row_table(e, nsteps, stream), ctypes.byref(table.s), e, int(n0),
-                       int(nsteps), _stream_ptr(stream)))
+            fn = self.lib.lens_te2d_step_rows if te else self.lib.lens_tm2d_step_rows
+            rows = self._row_table(e, nsteps, stream)
+            N.check(fn(ctypes.byref(self.s), rows, *span, int(n0), int(nsteps), _stream_ptr(stream)))
+            made += 2 if rows is not None else 0
         else:
-            fn = self.lib.lens_te2d_step_driven if self.pol == 's' else self.lib.lens_tm2d_step_driven
-            N.check(fn(ctypes.byref(self.s), ctypes.byref(table.s), e, ctypes.byref(drive.s), int(n0),
-                       int(nsteps), _stream_ptr(stream)))
+            fn = self.lib.lens_te2d_step_driven if te else self.lib.lens_tm2d_step_driven
+            N.check(fn(ctypes.byref(self.s), *span, d, int(n0), int(nsteps), _stream_ptr(stream)))
+        self.launches += made
 
     def _row_table(self, e, nsteps, stream):
         """The table of repeated coefficient rows for a span of nsteps, from the coefficients as

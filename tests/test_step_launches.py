@@ -1,0 +1,53 @@
+"""Launch counts of the step by step 2D spans (lens_te2d_step_launches / lens_tm2d_step_launches):
+host arithmetic on descriptors whose pointers are never followed."""
+import ctypes
+
+import pytest
+
+from lens_sensor_b200 import _native as N
+
+
+def _grid(pol, nx, ny, ptr=16):
+    g = N.TE2D() if pol == 's' else N.TM2D()
+    g.nx, g.ny, g.pitch = nx, ny, (ny + 31) // 32 * 32
+    for f in ('ez', 'hx', 'hy', 'ce_e', 'ce_h') if pol == 's' else ('ex', 'ey', 'hz', 'ca_x', 'ca_y'):
+        setattr(g, f, ptr)
+    for ax, n in ((g.ax, nx), (g.ay, ny)):
+        ax.e, ax.h = N.Profile(16, 16, 16, n, 0, 0), N.Profile(16, 16, 16, n - 1, 0, 0)
+    g.src = N.Source(-1, None, None, None, 0, 0, 0)
+    return g
+
+
+def _count(pol, nx, ny, epi=None, drive=False, n0=0, n=10, ptr=16):
+    lib = N.load()
+    fn = lib.lens_te2d_step_launches if pol == 's' else lib.lens_tm2d_step_launches
+    tab = N.StepTable(16, 16, 16, 16, 0, 100)
+    d = ctypes.byref(N.Drive2D()) if drive else None
+    return fn(ctypes.byref(_grid(pol, nx, ny, ptr)), ctypes.byref(tab), ctypes.byref(epi) if epi is not None else None, d, n0, n)
+
+
+def _epi(box=False, dft=None):
+    e = N.Epi2D()
+    e.iavg_n0 = 1 << 30
+    if box:
+        e.nbox, e.box_acc = 1, 16
+        e.box[0] = (ctypes.c_int * 4)(1, 9, 1, 9)
+    if dft:
+        e.dft, (e.dft_n0, e.dft_n1) = 16, dft
+    return e
+
+
+@pytest.mark.parametrize('pol,nx,ny,plain,box,window', [
+    ('s', 140, 96, 2, 2, 2), ('p', 140, 96, 2, 3, 3),           # one cell a thread; TM's epilogue is a launch
+    ('s', 3000, 400, 2, 3, 2), ('s', 8000, 300, 2, 3, 3),       # wide: boxes are a launch, and from 1.9 M cells TE's windows
+    ('p', 4000, 200, 2, 3, 3)])
+def test_launches_of_a_step(pol, nx, ny, plain, box, window):
+    assert _count(pol, nx, ny) == 10 * plain
+    assert _count(pol, nx, ny, _epi(box=True)) == 10 * box
+    assert _count(pol, nx, ny, _epi(dft=(4, 8))) == 6 * plain + 4 * window
+    assert _count(pol, nx, ny, _epi(dft=(4, 8)), n0=4, n=4) == 4 * window
+    one = 2 if pol == 's' else 3
+    assert _count(pol, nx, ny, _epi(box=True), drive=True) == 10 * one       # driven steps: one cell a thread
+    assert _count(pol, nx, ny, _epi(box=True), ptr=20) == 10 * one           # so with arrays off 16 bytes
+    assert _count(pol, nx, ny, n=0) == 0
+    assert _count(pol, nx, ny, n0=95) == -1                                  # beyond the table: refused
