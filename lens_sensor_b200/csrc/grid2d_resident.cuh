@@ -21,8 +21,8 @@
 // thread of the same columns polls them at the end of its next H phase until the
 // tag of the step it needs appears, so that the hop passes under the rest of both
 // phases.  Every poll is bounded; a wait that runs out sets *err, and all CTAs
-// leave the step loop at their next CTA barrier (or when they see *err), turn their
-// rows of the fields and sums into NaN, write them back and end.  Each slot of the halo rows is double-buffered by step
+// leave the step loop at their next CTA barrier (or when they see *err), write NaN
+// to their rows of the fields and sums and end.  Each slot of the halo rows is double-buffered by step
 // parity; a band publishes step n+1 only after it has read both neighbours' step n,
 // which they published after reading its step n-1, the slot's last content.
 //
@@ -883,10 +883,7 @@ __device__ __forceinline__ bool rs_loop(Th<RM> &t, const Band &B, const GPlan &p
             if (POL == 0) edge_out<RM, true>(xb, w, t.b, f2(0.f));
             else edge_out<RM, true>(xb, w, t.c, t.gc);
         }
-        if (__syncthreads_or(bad)) {  // one thread's wait ran out: the whole band's results are invalid
-            bad = true;
-            break;
-        }
+        if (__syncthreads_or(bad)) break;
 
         // ------------------------------------------------------------ E phase
         float x[EP];
@@ -907,6 +904,36 @@ __device__ __forceinline__ bool rs_loop(Th<RM> &t, const Band &B, const GPlan &p
         }
     }
     return bad;
+}
+
+// Columns j, j + 1 of a band whose results are invalid: NaN in the fields' own cells (what lies
+// beyond them stays as it is) and in every sum that the band feeds.  Apart from the band's code:
+// within it the steps' registers came out otherwise (TE 1201 x 431 in its windows 6.62 us a step
+// against 6.29).
+template <int POL>
+__device__ __noinline__ void rs_invalid(const GPlan &pl, const Band &B, int j, int *err) {
+    const float nan = __int_as_float(0x7fc00000);
+    const LensEpi2D &ep = pl.ep;
+    atomicOr(err, 1);
+    for (int r = 0; r < B.R; ++r) {
+        const int i = B.lo + r;
+        for (int c = j; c < j + 2 && c < B.ny; ++c) {
+            const size_t o = (size_t)i * B.P + c;
+            const bool h = i < B.nx - 1, v = c < B.ny - 1;
+            if (POL == 0 || h) B.f[0][o] = nan;
+            if (v) B.f[1][o] = nan;
+            if (h && (POL == 0 || v)) B.f[2][o] = nan;
+            float *const sum[3] = {ep.dft, ep.dft_ex, ep.dft_prev};
+            for (int q = 0; q < 3; ++q)
+                if (sum[q]) reinterpret_cast<float4 *>(sum[q])[o] = make_float4(nan, nan, nan, nan);
+            if (ep.iavg) ep.iavg[o] = nan;
+            for (int p = 0; p < ep.nplane; ++p)
+                for (int q = 0; q < 4; ++q)
+                    if (ep.plane[p] == i) ep.plane_acc[((size_t)p * 4 + q) * B.P + c] = nan;
+        }
+    }
+    for (int b = 0; b < ep.nbox; ++b)
+        if (ep.box[b][0] < B.lo + B.R && ep.box[b][1] > B.lo) atomicAdd(ep.box_acc + b, (double)nan);
 }
 
 // One band.  GEN: every warp in the general form (at most RM rows), else the lean forms.
@@ -1080,34 +1107,13 @@ __device__ __forceinline__ void rs_band(const GPlan &pl, const LensStepTable &ta
     else if (form == 0u) bad = rs_loop<RM, POL, 0u>(t, B, pl, tab, n0, nsteps, halo, err, prev, next, box, zb, hold, sdft, bacc);
     else if (form == V_N) bad = rs_loop<RM, POL, V_N>(t, B, pl, tab, n0, nsteps, halo, err, prev, next, box, zb, hold, sdft, bacc);
     else bad = rs_loop<RM, POL, V_N | V_Y>(t, B, pl, tab, n0, nsteps, halo, err, prev, next, box, zb, hold, sdft, bacc);
-    const LensEpi2D &ep = pl.ep;
-    if (bad) {  // the results are invalid: make that plain in the fields and in every sum of the band
-        const float nan = __int_as_float(0x7fc00000);
-        atomicOr(err, 1);
-#pragma unroll
-        for (int r = 0; r < RM; ++r) {  // the components' own cells: what lies beyond them stays as it is
-            const unsigned h = B.lo + r < B.nx - 1 ? ~0u : 0u, e = POL == 0 ? ~0u : h;
-            t.a[r] = bsel2(t.lt0 & e, t.lt1 & e, f2(nan), t.a[r]);
-            t.b[r] = bsel2(t.hx0, t.hx1, f2(nan), t.b[r]);
-            t.c[r] = bsel2(h & (POL == 0 ? t.lt0 : t.hx0), h & (POL == 0 ? t.lt1 : t.hx1), f2(nan), t.c[r]);
-        }
-        for (int b = 0; b < ep.nbox && box; ++b) bacc[b * 32 * W] = nan;
-        for (int r = 0; r < R; ++r)
-            for (int c = 0; c < 2; ++c) {
-                if (!lt[c]) continue;
-                const size_t o = (size_t)(B.lo + r) * B.P + j + c;
-                float *const sum[3] = {ep.dft, ep.dft_ex, ep.dft_prev};
-                for (int q = 0; q < 3; ++q)
-                    if (sum[q]) reinterpret_cast<float4 *>(sum[q])[o] = make_float4(nan, nan, nan, nan);
-                if (ep.iavg) ep.iavg[o] = nan;
-                for (int p = 0; p < ep.nplane; ++p)
-                    for (int q = 0; q < 4; ++q)
-                        if (ep.plane[p] == B.lo + r) ep.plane_acc[((size_t)p * 4 + q) * B.P + j + c] = nan;
-            }
+    if (__syncthreads_or(bad)) {  // one thread's wait ran out: the whole band's results are invalid
+        rs_invalid<POL>(pl, B, j, err);
+        return;
     }
 
     // ---- state out
-    if (hold && !bad && lt[0])
+    if (hold && lt[0])
         for (int r = 0; r < R; ++r) {
             const float4 *l = reinterpret_cast<const float4 *>(sdft) + (size_t)r * NS;
             gdft[(size_t)r * B.P] = l[0];

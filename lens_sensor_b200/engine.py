@@ -250,12 +250,14 @@ class Grid2D:
         self.rs_scratch = torch.empty(need, dtype=torch.uint8, device=dev) if need else None
         self.rs_err = torch.zeros(1, dtype=torch.int32, device=dev) if need else None
         self.rs_stream = None       # stream of the last resident launch
-        self.rs_plan = None         # rows, threads and bands of that launch
+        self.rs_plan = None         # rows, threads and bands of that launch; steps from which by sums, their most
         if need:
             plan = [ctypes.c_int() for _ in range(3)]
             fn = self.lib.lens_te2d_resident_rows if self.pol == 's' else self.lib.lens_tm2d_resident_rows
             N.check(fn(ctypes.byref(self.s), 0, *map(ctypes.byref, plan)))
             self.rs_plan = tuple(v.value for v in plan)
+            self.rs_steps = [resident_steps(self.pol, *self.rs_plan, q) for q in range(5)]
+            self.rs_most = max(self.rs_steps)
         # row table of the wide passes (lens_te2d_row_table), formed anew by every step() that reads it
         self.rowref = torch.empty(nx, dtype=torch.int32, device=dev) if not need else None
 
@@ -284,14 +286,15 @@ class Grid2D:
 
     def step(self, table, n0, nsteps, epi=None, stream=None, drive=None):
         e = ctypes.byref(epi.s) if epi is not None else None
-        if drive is None and self.rs_scratch is not None and nsteps >= RS_MIN_STEPS and \
-                nsteps >= resident_steps(self.pol, *self.rs_plan, sums_a_step(epi.s, int(n0), int(nsteps)) if epi else 0):
+        if drive is None and self.rs_scratch is not None and nsteps >= RS_MIN_STEPS and (
+                nsteps >= self.rs_most or nsteps >= self.rs_steps[sums_a_step(epi.s, int(n0), int(nsteps)) if epi else 0]):
             fn = self.lib.lens_te2d_resident if self.pol == 's' else self.lib.lens_tm2d_resident
+            on = stream if stream is not None else torch.cuda.current_stream()
             st = fn(ctypes.byref(self.s), ctypes.byref(table.s), e, int(n0), int(nsteps), _ptr(self.rs_scratch),
-                    self.rs_scratch.numel(), _ptr(self.rs_err), _stream_ptr(stream))
+                    self.rs_scratch.numel(), _ptr(self.rs_err), _stream_ptr(on))
             if st != N.ERR_SIZE:      # else: a call that only the steps below carry
                 self.launches += 1
-                self.rs_stream = stream if stream is not None else torch.cuda.current_stream()
+                self.rs_stream = on
                 return N.check(st)
         te = self.pol == 's'
         d = ctypes.byref(drive.s) if drive is not None else None
