@@ -235,9 +235,16 @@ constexpr int RS_RX = 2;                      // rows of a band in the general f
 // Floats of one warp's edge column: rows 0..RM-1 and the ghost row RM.
 constexpr int rs_edge(int rm) { return (rm + 1 + 3) / 4 * 4; }
 
-// Row pitch of the y psi in shared memory: the strip columns' slots, then a pair per
-// lane for columns outside the strips (stays 0: b = c = 0 there).
-constexpr int RS_YP = RS_MAXWY + 64;
+// Row pitch of the y psi in shared memory: a slot pair for every thread's columns that
+// meet a strip (a strip end may split a pair at either side), then a pair per lane for
+// columns outside the strips, whose psi stays 0.
+constexpr int RS_YD = RS_MAXWY + 4, RS_YP = RS_YD + 64;
+
+// Slot pair of columns j, j + 1 (j even): st, strip indices of the two.
+__device__ __forceinline__ int rs_yslot(const int (&st)[2], const LensProfile &p, int j, int lane) {
+    if (st[0] < 0 && st[1] < 0) return RS_YD + 2 * lane;
+    return j < p.lo ? j : (p.lo + 1) / 2 * 2 + j - (p.n - p.hi) / 2 * 2;
+}
 
 // Rows of a phase.  A band of the lean forms fills its template or lacks up to
 // RS_SPARE rows (tested for); the general form tests every row, which keeps the rows'
@@ -263,10 +270,11 @@ struct Th {
     // column tests as bit masks: j < ny-1, j < ny, 0 < j < ny-1, zero after the E update
     // (TE: a PEC face or beyond ny; TM Ex: a PEC face); source column
     unsigned hx0, hx1, lt0, lt1, in0, in1, ze0, ze1;
+    unsigned sh0, sh1, se0, se1;     // columns of a y strip (H, E)
     bool sr0, sr1;
     const float *cs;                 // coefficient rows, at this thread's columns
     float *xh, *xe;                  // x psi rows, at this thread's columns
-    float *yh0, *yh1, *ye0, *ye1;    // y psi slots of row 0 (rows RS_YP apart)
+    float *yh, *ye;                  // y psi slots of row 0 (rows RS_YP apart)
     const RowC *rowc;                // rows 0..RM-1 and the ghost row RM
     int NS, xs;                      // row pitch of the shared arrays; of the x psi rows (0: a column beyond them)
 };
@@ -346,21 +354,26 @@ __device__ __forceinline__ void h_load(const Th<RM> &t, int r, RowIn &n) {
     } else if (V & V_N) {
         n.kx = t.rowc[r].kxh;
     }
-    if (V & V_Y) n.y = make_float2(t.yh0[r * RS_YP], t.yh1[r * RS_YP]);
+    if (V & V_Y) n.y = ld2(t.yh + r * RS_YP);
 }
 
 template <int RM, int POL, unsigned V>
 __device__ __forceinline__ void h_store(const Th<RM> &t, int r, const RowIn &n) {
     if (V & V_X) st2(t.xh + r * t.xs, n.x);
-    if (V & V_Y) {
-        t.yh0[r * RS_YP] = n.y.x;
-        t.yh1[r * RS_YP] = n.y.y;
-    }
+    if (V & V_Y) st2(t.yh + r * RS_YP, n.y);
 }
 
-// psi' kept where the masks say, d * kx + psi' returned.
-__device__ __forceinline__ float2 psi_x(RowIn &n, float2 d, unsigned m0, unsigned m1) {
-    const float2 p = cell_psi(f2(n.bx), n.x, f2(n.cx), d);
+// Kept in a column or row of a strip, 0 outside, where psi is 0 whatever d: c = 0 alone would
+// make it NaN of an infinite d, and the slot that the columns outside share with it.  Of the
+// products (as here), of d and of psi, the y mask cost the warps at the y faces 0.7, 0.6 and
+// 1.1 % over 36 sizes, their psi in slot pairs (5 % as single slots, the masks then needed
+// registers that there were not).
+__device__ __forceinline__ float2 in_strip(unsigned m0, unsigned m1, float2 v) { return bsel2(m0, m1, v, f2(0.f)); }
+
+// psi' kept where the masks say, d * kx + psi' returned.  strip: the row lies in its strip.
+__device__ __forceinline__ float2 psi_x(RowIn &n, float2 d, unsigned m0, unsigned m1, bool strip) {
+    const unsigned s = strip ? ~0u : 0u;
+    const float2 p = in_strip(s, s, cell_psi(f2(n.bx), n.x, f2(n.cx), d));
     n.x = bsel2(m0, m1, p, n.x);
     return fma2(d, f2(n.kx), p);
 }
@@ -375,7 +388,7 @@ __device__ __forceinline__ void h_row(Th<RM> &t, int r, float edge, RowIn &n) {
         const float2 ez = t.a[r], d = sub2(pair_up(ez, t.lane, edge), ez);
         float2 u;
         if (V & V_Y) {
-            n.y = cell_psi(t.byh, n.y, t.cyh, d);
+            n.y = fma2(t.byh, n.y, in_strip(t.sh0, t.sh1, mul2(t.cyh, d)));
             u = fma2(d, t.kyh, n.y);
         } else {
             u = mul2(d, t.kyh);
@@ -385,7 +398,7 @@ __device__ __forceinline__ void h_row(Th<RM> &t, int r, float edge, RowIn &n) {
         if (r + 1 < RM) {
             const float2 e = sub2(t.a[rn], ez);
             const unsigned m0 = hok ? t.lt0 : 0u, m1 = hok ? t.lt1 : 0u;
-            const float2 v = (V & V_X) ? psi_x(n, e, m0, m1) : mul2(e, f2(n.kx));
+            const float2 v = (V & V_X) ? psi_x(n, e, m0, m1, n.f & R_XH) : mul2(e, f2(n.kx));
             const float2 hy = fma2(f2(t.ch), v, t.c[r]);
             if (V & V_Y) t.c[r] = bsel2(m0, m1, hy, t.c[r]);
             else t.c[r] = sel2(hok, hok, hy, t.c[r]);
@@ -393,10 +406,10 @@ __device__ __forceinline__ void h_row(Th<RM> &t, int r, float edge, RowIn &n) {
     } else if (r + 1 < RM) {
         const float2 ex = t.a[r], dyx = sub2(t.b[rn], t.b[r]), dxy = sub2(pair_up(ex, t.lane, edge), ex);
         const unsigned m0 = hok ? t.hx0 : 0u, m1 = hok ? t.hx1 : 0u;
-        const float2 u = (V & V_X) ? psi_x(n, dyx, m0, m1) : mul2(dyx, f2(n.kx));
+        const float2 u = (V & V_X) ? psi_x(n, dyx, m0, m1, n.f & R_XH) : mul2(dyx, f2(n.kx));
         float2 v;
         if (V & V_Y) {
-            const float2 py = cell_psi(t.byh, n.y, t.cyh, dxy);
+            const float2 py = fma2(t.byh, n.y, in_strip(t.sh0, t.sh1, mul2(t.cyh, dxy)));
             n.y = sel2(hok, hok, py, n.y);
             v = fma2(dxy, t.kyh, py);
         } else {
@@ -416,7 +429,7 @@ __device__ __forceinline__ void h_last(Th<RM> &t, int r, float2 en, float edge) 
     const bool hok = !(V & V_X) || (n.f & R_HOK);
     const float2 d = sub2(en, POL == 0 ? t.a[r] : t.b[r]);
     const unsigned m0 = hok ? (POL == 0 ? t.lt0 : t.hx0) : 0u, m1 = hok ? (POL == 0 ? t.lt1 : t.hx1) : 0u;
-    const float2 u = (V & V_X) ? psi_x(n, d, m0, m1) : mul2(d, f2(n.kx));
+    const float2 u = (V & V_X) ? psi_x(n, d, m0, m1, n.f & R_XH) : mul2(d, f2(n.kx));
     float2 h;
     if (POL == 0) {
         h = fma2(f2(t.ch), u, t.c[r]);
@@ -424,7 +437,7 @@ __device__ __forceinline__ void h_last(Th<RM> &t, int r, float2 en, float edge) 
         const float2 ex = t.a[r], dxy = sub2(pair_up(ex, t.lane, edge), ex);
         float2 v;
         if (V & V_Y) {
-            const float2 py = cell_psi(t.byh, n.y, t.cyh, dxy);
+            const float2 py = fma2(t.byh, n.y, in_strip(t.sh0, t.sh1, mul2(t.cyh, dxy)));
             n.y = sel2(hok, hok, py, n.y);
             v = fma2(dxy, t.kyh, py);
         } else {
@@ -442,7 +455,8 @@ __device__ __forceinline__ void h_last(Th<RM> &t, int r, float2 en, float edge) 
 template <int RM, int POL, unsigned V>
 __device__ __forceinline__ void h_ghost(Th<RM> &t, float2 ep, float edge) {
     const RowC &rc = t.rowc[RM];
-    const float2 d = sub2(POL == 0 ? t.a[0] : t.b[0], ep), px = cell_psi(f2(rc.bxh), t.gpx, f2(rc.cxh), d);
+    const unsigned s = rc.flags & R_XH ? ~0u : 0u;
+    const float2 d = sub2(POL == 0 ? t.a[0] : t.b[0], ep), px = in_strip(s, s, cell_psi(f2(rc.bxh), t.gpx, f2(rc.cxh), d));
     const float2 u = fma2(d, f2(rc.kxh), px);
     const unsigned m0 = POL == 0 ? t.lt0 : t.hx0, m1 = POL == 0 ? t.lt1 : t.hx1;
     float2 h;
@@ -452,7 +466,7 @@ __device__ __forceinline__ void h_ghost(Th<RM> &t, float2 ep, float edge) {
         const float2 dxy = sub2(pair_up(t.ga, t.lane, edge), t.ga);
         float2 v;
         if (V & V_Y) {
-            t.gph = cell_psi(t.byh, t.gph, t.cyh, dxy);
+            t.gph = fma2(t.byh, t.gph, in_strip(t.sh0, t.sh1, mul2(t.cyh, dxy)));
             v = fma2(dxy, t.kyh, t.gph);
         } else {
             v = mul2(dxy, t.kyh);
@@ -469,7 +483,7 @@ __device__ __forceinline__ void e_ghost(Th<RM> &t, float edge) {
     const float2 d = sub2(t.gc, pair_dn(t.gc, t.lane, edge));
     float2 u;
     if (V & V_Y) {
-        t.gpe = cell_psi(t.bye, t.gpe, t.cye, d);
+        t.gpe = fma2(t.bye, t.gpe, in_strip(t.se0, t.se1, mul2(t.cye, d)));
         u = fma2(d, t.kye, t.gpe);
     } else {
         u = mul2(d, t.kye);
@@ -510,7 +524,7 @@ __device__ __forceinline__ void e_load(const Th<RM> &t, int r, RowIn &n) {
     } else if (V & V_N) {
         n.kx = t.rowc[r].kxe;
     }
-    if (V & V_Y) n.y = make_float2(t.ye0[r * RS_YP], t.ye1[r * RS_YP]);
+    if (V & V_Y) n.y = ld2(t.ye + r * RS_YP);
     n.k0 = t.k0;
     n.k1 = t.k1;
     n.k2 = t.k2;
@@ -529,10 +543,7 @@ __device__ __forceinline__ void e_load(const Th<RM> &t, int r, RowIn &n) {
 template <int RM, int POL, unsigned V>
 __device__ __forceinline__ void e_store(const Th<RM> &t, int r, const RowIn &n) {
     if (V & V_X) st2(t.xe + r * t.xs, n.x);
-    if (V & V_Y) {
-        t.ye0[r * RS_YP] = n.y.x;
-        t.ye1[r * RS_YP] = n.y.y;
-    }
+    if (V & V_Y) st2(t.ye + r * RS_YP, n.y);
 }
 
 // E of row r at table row k; hm: the H field of row i-1 (TE Hy, TM Hz).
@@ -542,10 +553,10 @@ __device__ __forceinline__ void e_row(Th<RM> &t, int r, float2 hm, float edge, R
     const bool rin = rf & R_IN;
     if (POL == 0) {
         const float2 hx = t.b[r], dhy = sub2(t.c[r], hm), dhx = sub2(hx, pair_dn(hx, t.lane, edge));
-        float2 u = (V & V_X) ? psi_x(n, dhy, t.in0, t.in1) : mul2(dhy, f2(n.kx));
+        float2 u = (V & V_X) ? psi_x(n, dhy, t.in0, t.in1, rf & R_XE) : mul2(dhy, f2(n.kx));
         u = fma2(neg2(dhx), t.kye, u);
         if (V & V_Y) {
-            const float2 py = cell_psi(t.bye, n.y, t.cye, dhx);
+            const float2 py = fma2(t.bye, n.y, in_strip(t.se0, t.se1, mul2(t.cye, dhx)));
             n.y = sel2(rin, rin, py, n.y);
             u = sub2(u, py);
         }
@@ -561,14 +572,14 @@ __device__ __forceinline__ void e_row(Th<RM> &t, int r, float2 hm, float edge, R
         const float2 hz = t.c[r], d = sub2(hz, pair_dn(hz, t.lane, edge)), d2 = sub2(hz, hm);
         float2 u;
         if (V & V_Y) {
-            const float2 py = cell_psi(t.bye, n.y, t.cye, d);
+            const float2 py = fma2(t.bye, n.y, in_strip(t.se0, t.se1, mul2(t.cye, d)));
             const bool on = rf & R_HOK;
             n.y = sel2(on, on, py, n.y);
             u = fma2(d, t.kye, py);
         } else {
             u = mul2(d, t.kye);
         }
-        const float2 v = (V & V_X) ? psi_x(n, d2, t.hx0, t.hx1) : mul2(d2, f2(n.kx));
+        const float2 v = (V & V_X) ? psi_x(n, d2, t.hx0, t.hx1, rf & R_XE) : mul2(d2, f2(n.kx));
         // Ex at (i+1/2, j) (boundaries.py:249-258)
         float2 e = t.lossy ? mul2(t.a[r], n.k2) : t.a[r];
         const float2 en = fma2(n.k0, u, e);
@@ -986,7 +997,6 @@ __device__ __forceinline__ void rs_band(const GPlan &pl, const LensStepTable &ta
     // per column: tests, 1/kappa_y, y-psi slot and its profile values
     bool hx[2], lt[2], in[2], pe[2], sr[2];
     float kyh[2], kye[2], bh[2], chh[2], be[2], ce[2];
-    float *qh[2], *qe[2];
     int sjh[2], sje[2];
 #pragma unroll
     for (int c = 0; c < 2; ++c) {
@@ -1004,18 +1014,18 @@ __device__ __forceinline__ void rs_band(const GPlan &pl, const LensStepTable &ta
         chh[c] = sjh[c] >= 0 ? ypc[RS_MAXWY + sjh[c]] : 0.f;
         be[c] = sje[c] >= 0 ? ypc[2 * RS_MAXWY + sje[c]] : 0.f;
         ce[c] = sje[c] >= 0 ? ypc[3 * RS_MAXWY + sje[c]] : 0.f;
-        qh[c] = yps_h + (sjh[c] >= 0 ? sjh[c] : RS_MAXWY + 2 * lane + c);
-        qe[c] = yps_e + (sje[c] >= 0 ? sje[c] : RS_MAXWY + 2 * lane + c);
     }
     t.kyh = make_float2(kyh[0], kyh[1]); t.kye = make_float2(kye[0], kye[1]);
     t.byh = make_float2(bh[0], bh[1]); t.cyh = make_float2(chh[0], chh[1]);
     t.bye = make_float2(be[0], be[1]); t.cye = make_float2(ce[0], ce[1]);
-    t.yh0 = qh[0]; t.yh1 = qh[1]; t.ye0 = qe[0]; t.ye1 = qe[1];
+    t.yh = yps_h + rs_yslot(sjh, gp->ay.h, j, lane);
+    t.ye = yps_e + rs_yslot(sje, gp->ay.e, j, lane);
     auto mask = [](bool v) { return v ? ~0u : 0u; };
     t.hx0 = mask(hx[0]); t.hx1 = mask(hx[1]); t.lt0 = mask(lt[0]); t.lt1 = mask(lt[1]);
     t.in0 = mask(in[0]); t.in1 = mask(in[1]);
     t.ze0 = mask(pe[0] || (POL == 0 && !lt[0])); t.ze1 = mask(pe[1] || (POL == 0 && !lt[1]));
     t.sr0 = sr[0]; t.sr1 = sr[1];
+    t.sh0 = mask(sjh[0] >= 0); t.sh1 = mask(sjh[1] >= 0); t.se0 = mask(sje[0] >= 0); t.se1 = mask(sje[1] >= 0);
     // the row form of this warp
     bool same = !GEN;
     const RowC r0 = rowc[0];
@@ -1056,8 +1066,8 @@ __device__ __forceinline__ void rs_band(const GPlan &pl, const LensStepTable &ta
             if (GEN && se >= 0 && on) st2(t.xe + r * NS, in2(B.pxe + (size_t)se * B.P + j));
 #pragma unroll
             for (int c = 0; c < 2; ++c) {
-                if (sjh[c] >= 0) yps_h[r * RS_YP + sjh[c]] = B.pyh[(size_t)(B.lo + r) * B.wyh + sjh[c]];
-                if (sje[c] >= 0) yps_e[r * RS_YP + sje[c]] = B.pye[(size_t)(B.lo + r) * B.wye + sje[c]];
+                if (sjh[c] >= 0) t.yh[r * RS_YP + c] = B.pyh[(size_t)(B.lo + r) * B.wyh + sjh[c]];
+                if (sje[c] >= 0) t.ye[r * RS_YP + c] = B.pye[(size_t)(B.lo + r) * B.wye + sje[c]];
             }
         }
     }
@@ -1138,8 +1148,8 @@ __device__ __forceinline__ void rs_band(const GPlan &pl, const LensStepTable &ta
             if (GEN && se >= 0 && lt[0]) out2(B.pxe + (size_t)se * B.P + j, ld2(t.xe + r * NS));
 #pragma unroll
             for (int c = 0; c < 2; ++c) {
-                if (sjh[c] >= 0) B.pyh[(size_t)(B.lo + r) * B.wyh + sjh[c]] = yps_h[r * RS_YP + sjh[c]];
-                if (sje[c] >= 0) B.pye[(size_t)(B.lo + r) * B.wye + sje[c]] = yps_e[r * RS_YP + sje[c]];
+                if (sjh[c] >= 0) B.pyh[(size_t)(B.lo + r) * B.wyh + sjh[c]] = t.yh[r * RS_YP + c];
+                if (sje[c] >= 0) B.pye[(size_t)(B.lo + r) * B.wye + sje[c]] = t.ye[r * RS_YP + c];
             }
         }
     }
