@@ -279,7 +279,8 @@ int run(const LensInst2D &g, const LensEpi2D *ep, const LensStepTable *tab, int 
     // the node DFT's sums sit in shared memory where that leaves every CTA resident
     const void *kern = p.form->kernel(p.wide);
     size_t sm = rs_smem(*p.form, p.ncol, p.nc, e.nbox, false);
-    if (e.dft && e.dft_n0 < n0 + nsteps && e.dft_n1 > n0) {
+    // (not where another sum runs on the same array: that one is added to in global memory)
+    if (e.dft && e.dft != e.dft_prev && e.dft != e.dft_ex && e.dft_n0 < n0 + nsteps && e.dft_n1 > n0) {
         int dev = 0, smax = 0, nsm = 0, per = 0;
         const size_t smd = rs_smem(*p.form, p.ncol, p.nc, e.nbox, true);
         if (cudaGetDevice(&dev) == cudaSuccess &&
