@@ -892,7 +892,8 @@ int te2d_run(const LensTE2D *g, const LensStepTable *tab, const LensEpi2D *ep, c
     if (!grid2d_ok(g) || !psi2d_ok(g) || !g->ez || !g->hx || !g->hy || !g->ce_e || !g->ce_h || nsteps < 0 ||
         !lens_table_ok(tab, n0, nsteps) || !epi2d_ok(ep, tab, g->nx) || !drive2d_ok(dr, tab, g->nx))
         return LENS_ERR_ARG;
-    const LensEpi2D e = ep ? *ep : empty_epi();
+    LensEpi2D e = ep ? *ep : empty_epi();
+    lens_clip_boxes(e, g->nx, g->ny);
     const LensDrive2D d = dr ? *dr : LensDrive2D{};
     cudaStream_t s = static_cast<cudaStream_t>(stream);
     const Launch go{count};
@@ -925,7 +926,8 @@ int tm2d_run(const LensTM2D *g, const LensStepTable *tab, const LensEpi2D *ep, c
         (!g->da_x) != (!g->da_y) || nsteps < 0 || !lens_table_ok(tab, n0, nsteps) ||
         !epi2d_ok(ep, tab, g->nx) || !drive2d_ok(dr, tab, g->nx))
         return LENS_ERR_ARG;
-    const LensEpi2D e = ep ? *ep : empty_epi();
+    LensEpi2D e = ep ? *ep : empty_epi();
+    lens_clip_boxes(e, g->nx, g->ny);
     const LensDrive2D d = dr ? *dr : LensDrive2D{};
     cudaStream_t s = static_cast<cudaStream_t>(stream);
     const Launch go{count};

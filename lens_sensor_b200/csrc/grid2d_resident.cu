@@ -253,6 +253,7 @@ int run(const LensInst2D &g, const LensEpi2D *ep, const LensStepTable *tab, int 
     if (e.dft_raw || e.ex2 || e.nsx != 0 || e.nbox < 0 || e.nbox > LENS_MAX_BOX || (e.nbox > 0 && !e.box_acc) ||
         e.nplane < 0 || e.nplane > LENS_MAX_PLANE || (e.nplane > 0 && !e.plane_acc) || (e.dft_ex && g.pol == 0))
         return LENS_ERR_SIZE;
+    lens_clip_boxes(pl.ep, g.nx, g.ny);
     for (int q = 0; q < e.nplane; ++q)
         if (e.plane[q] < 1 || e.plane[q] > g.nx - 2) return LENS_ERR_SIZE;
     if ((e.dft || e.dft_ex || e.dft_prev || e.nplane > 0) && (!tab->pe || !tab->ph)) return LENS_ERR_SIZE;

@@ -62,6 +62,16 @@ static inline bool lens_table_ok(const LensStepTable *t, int n0, int nsteps) {
     return t && t->wt && t->env && n0 >= t->t0 && (n0 + nsteps) <= (t->t0 + t->n_table);
 }
 
+// Detector boxes cut to the grid: the same nodes, in numbers that sums and differences of
+// row and column indices cannot run over.
+static inline void lens_clip_boxes(LensEpi2D &e, int nx, int ny) {
+    for (int b = 0; b < e.nbox; ++b)
+        for (int q = 0; q < 4; ++q) {
+            const int n = q < 2 ? nx : ny;
+            e.box[b][q] = e.box[b][q] < 0 ? 0 : (e.box[b][q] > n ? n : e.box[b][q]);
+        }
+}
+
 static inline int lens_cuda_status(void) {
     return cudaGetLastError() == cudaSuccess ? LENS_OK : LENS_ERR_CUDA;
 }

@@ -39,3 +39,27 @@ def test_two_windows_on_one_array(pol, windows):
         torch.cuda.synchronize()
         out.append(ep.dft)
     assert bool(out[1].any()) and torch.equal(*out)
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize('size', [('s', 140, 96), ('p', 140, 96), ('s', 3001, 401), ('p', 2703, 300)])
+@pytest.mark.parametrize('resident', [True, False])
+def test_boxes_beyond_the_grid(size, resident, monkeypatch):
+    """Box ends anywhere in an int: the nodes of the grid that lie between them, none where they cross."""
+    import torch
+    from lens_sensor_b200 import engine as E
+    pol, nx, ny = size
+    lo, hi = -2 ** 31, 2 ** 31 - 1
+    a, b = (_grid(pol, nx, ny, True, 5) for _ in range(2))
+    tab = _tab(a, 6)
+    monkeypatch.setattr(E, 'RS_MIN_STEPS', 4 if resident else 1 << 30)
+    boxes = [(lo, 40, lo, hi), (10, lo, 0, ny), (nx - 9, hi, -5, ny + 5), (hi, lo, hi, lo)]
+    ea, eb = E.Epi2D(a, boxes=boxes), E.Epi2D(b, boxes=[(0, 40, 0, ny), (0, 0, 0, 0), (nx - 9, nx, 0, ny), (0, 0, 0, 0)])
+    a.step(tab, 7, 6, ea)
+    _one_cell(b, tab, 7, 6, eb)
+    torch.cuda.synchronize()
+    x, y = ea.box_acc, eb.box_acc
+    assert float(y[0]) > 0 and float(y[2]) > 0 and float(y[1]) == float(y[3]) == 0
+    assert float((x - y).abs().max()) <= 1e-12 * float(y.abs().max())
+    for q in FIELDS[pol]:
+        assert torch.equal(getattr(a, q), getattr(b, q)), q
