@@ -51,7 +51,6 @@
 namespace {
 
 constexpr int RS_MAXW = 12;                  // warps per CTA, 64 columns each: ny <= 768
-constexpr int RS_MAXNY = 64 * RS_MAXW;
 constexpr int RS_MAXWY = 64;                 // psi strip width of one y staggering (lo + hi)
 constexpr unsigned RS_TRIES = 1u << 22;    // polls per wait (each an L2 round trip, >= 0.3 us)
 constexpr unsigned FULL = 0xffffffffu;
@@ -230,7 +229,6 @@ __device__ __forceinline__ void band_setup(const LensInst2D *gp, const GPlan &pl
 // Forms of a row (see the top of the file).
 enum : unsigned { V_N = 1u, V_Y = 2u, V_X = 4u };
 constexpr unsigned V_GEN = V_N | V_Y | V_X;
-constexpr int RS_RX = 2;                      // rows of a band in the general form
 
 // Floats of one warp's edge column: rows 0..RM-1 and the ghost row RM.
 constexpr int rs_edge(int rm) { return (rm + 1 + 3) / 4 * 4; }
