@@ -1472,7 +1472,7 @@ int make_chunks(const LensGrid3D *g, int target, int *x, int *strip) {
     int lo = g->ax.h.lo > g->ax.e.lo ? g->ax.h.lo : g->ax.e.lo;
     int hi = nx - 1 - g->ax.h.hi;
     if (nx - g->ax.e.hi < hi) hi = nx - g->ax.e.hi;
-    lo = lo > 0 ? lo + 1 : 0;  // the next chunk's warm-up plane lo must be strip-free too
+    lo = lo > 0 ? std::min(lo + 1, nx) : 0;  // the next chunk's warm-up plane lo must be strip-free too
     if (hi < lo) hi = lo;
     auto add = [&](int a, int b, int s) {
         if (b <= a || n >= MAXCH) return;
