@@ -184,6 +184,13 @@ int lens_te2d_step_driven(const LensTE2D *g, const LensStepTable *tab, const Len
 int lens_tm2d_step_driven(const LensTM2D *g, const LensStepTable *tab, const LensEpi2D *ep,
                           const LensDrive2D *drive, int n0, int nsteps, void *stream);
 
+/* Any of the three (rowref, drive: NULL where not wanted), adding the kernel launches
+ * made to *launches (NULL: not counted).                                      */
+int lens_te2d_step_counted(const LensTE2D *g, const int *rowref, const LensStepTable *tab, const LensEpi2D *ep,
+                           const LensDrive2D *drive, int n0, int nsteps, int *launches, void *stream);
+int lens_tm2d_step_counted(const LensTM2D *g, const int *rowref, const LensStepTable *tab, const LensEpi2D *ep,
+                           const LensDrive2D *drive, int n0, int nsteps, int *launches, void *stream);
+
 /* Kernel launches that lens_*_step, lens_*_step_rows (drive NULL) or lens_*_step_driven
  * makes for a span, or < 0 where the call is refused.  Nothing is launched.   */
 int lens_te2d_step_launches(const LensTE2D *g, const LensStepTable *tab, const LensEpi2D *ep, const LensDrive2D *drive,

@@ -138,6 +138,10 @@ SIGNATURES = {
     'lens_tm2d_step': (c_int, [POINTER(TM2D), POINTER(StepTable), POINTER(Epi2D), c_int, c_int, c_void_p]),
     'lens_te2d_step_rows': (c_int, [POINTER(TE2D), c_void_p, POINTER(StepTable), POINTER(Epi2D), c_int, c_int, c_void_p]),
     'lens_tm2d_step_rows': (c_int, [POINTER(TM2D), c_void_p, POINTER(StepTable), POINTER(Epi2D), c_int, c_int, c_void_p]),
+    'lens_te2d_step_counted': (c_int, [POINTER(TE2D), c_void_p, POINTER(StepTable), POINTER(Epi2D), POINTER(Drive2D), c_int,
+                                       c_int, POINTER(c_int), c_void_p]),
+    'lens_tm2d_step_counted': (c_int, [POINTER(TM2D), c_void_p, POINTER(StepTable), POINTER(Epi2D), POINTER(Drive2D), c_int,
+                                       c_int, POINTER(c_int), c_void_p]),
     'lens_te2d_step_launches': (c_int, [POINTER(TE2D), POINTER(StepTable), POINTER(Epi2D), POINTER(Drive2D), c_int, c_int]),
     'lens_tm2d_step_launches': (c_int, [POINTER(TM2D), POINTER(StepTable), POINTER(Epi2D), POINTER(Drive2D), c_int, c_int]),
     'lens_te2d_row_table': (c_int, [POINTER(TE2D), POINTER(Epi2D), c_int, c_void_p, c_void_p]),

@@ -877,18 +877,20 @@ dim3 box_grid(const LensEpi2D &e, int nx, int ny) {
     return w > 0 && h > 0 ? dim3((w + BX - 1) / BX, (h + BY * BOXR - 1) / (BY * BOXR), e.nbox) : dim3(0, 1, 1);
 }
 
-// The launches of a span, made or (count) only counted.
+// The launches of a span, made or (dry) only counted.
 struct Launch {
-    int *count;
+    int *count;  // or NULL
+    bool dry;
     template <class F>
     void operator()(F launch) const {
         if (count) ++*count;
-        else launch();
+        if (!dry) launch();
     }
 };
 
 int te2d_run(const LensTE2D *g, const LensStepTable *tab, const LensEpi2D *ep, const LensDrive2D *dr, int n0,
-             int nsteps, void *stream, const int *rowref = nullptr, int *count = nullptr) {
+             int nsteps, void *stream, const int *rowref = nullptr, int *count = nullptr,
+             bool dry = false) {
     if (!grid2d_ok(g) || !psi2d_ok(g) || !g->ez || !g->hx || !g->hy || !g->ce_e || !g->ce_h || nsteps < 0 ||
         !lens_table_ok(tab, n0, nsteps) || !epi2d_ok(ep, tab, g->nx) || !drive2d_ok(dr, tab, g->nx))
         return LENS_ERR_ARG;
@@ -896,7 +898,7 @@ int te2d_run(const LensTE2D *g, const LensStepTable *tab, const LensEpi2D *ep, c
     lens_clip_boxes(e, g->nx, g->ny);
     const LensDrive2D d = dr ? *dr : LensDrive2D{};
     cudaStream_t s = static_cast<cudaStream_t>(stream);
-    const Launch go{count};
+    const Launch go{count, dry};
     const dim3 blk(BX, BY), grd((g->ny + BX - 1) / BX, (g->nx + BY - 1) / BY);
     const double cells = (double)g->nx * g->ny;
     if (cells >= WIDE_TE && wide_ok(e, dr, {g->ez, g->hx, g->hy, g->ce_e, g->ce_h})) {
@@ -911,17 +913,18 @@ int te2d_run(const LensTE2D *g, const LensStepTable *tab, const LensEpi2D *ep, c
             if (epi2d_beyond_boxes(&e, n)) go([&] { te2d_epi<<<grd, blk, 0, s>>>(*g, *tab, e, n); });
             else if (bg.x > 0) go([&] { box2d<<<bg, blk, 0, s>>>(*g, e); });
         }
-        return count ? LENS_OK : lens_cuda_status();
+        return dry ? LENS_OK : lens_cuda_status();
     }
     for (int n = n0; n < n0 + nsteps; ++n) {
         go([&] { te2d_h<<<grd, blk, 0, s>>>(*g); });
         go([&] { te2d_e<<<grd, blk, 0, s>>>(*g, *tab, e, n, d); });
     }
-    return count ? LENS_OK : lens_cuda_status();
+    return dry ? LENS_OK : lens_cuda_status();
 }
 
 int tm2d_run(const LensTM2D *g, const LensStepTable *tab, const LensEpi2D *ep, const LensDrive2D *dr, int n0,
-             int nsteps, void *stream, const int *rowref = nullptr, int *count = nullptr) {
+             int nsteps, void *stream, const int *rowref = nullptr, int *count = nullptr,
+             bool dry = false) {
     if (!grid2d_ok(g) || !psi2d_ok(g) || !g->ex || !g->ey || !g->hz || !g->ca_x || !g->ca_y ||
         (!g->da_x) != (!g->da_y) || nsteps < 0 || !lens_table_ok(tab, n0, nsteps) ||
         !epi2d_ok(ep, tab, g->nx) || !drive2d_ok(dr, tab, g->nx))
@@ -930,7 +933,7 @@ int tm2d_run(const LensTM2D *g, const LensStepTable *tab, const LensEpi2D *ep, c
     lens_clip_boxes(e, g->nx, g->ny);
     const LensDrive2D d = dr ? *dr : LensDrive2D{};
     cudaStream_t s = static_cast<cudaStream_t>(stream);
-    const Launch go{count};
+    const Launch go{count, dry};
     const dim3 blk(BX, BY), grd((g->ny + BX - 1) / BX, (g->nx + BY - 1) / BY);
     if ((double)g->nx * g->ny >= WIDE_TM && wide_ok(e, dr, {g->ex, g->ey, g->hz, g->ca_x, g->ca_y, g->da_x, g->da_y})) {
         const dim3 wb(BX, WT), wg((g->ny + BX * WV - 1) / (BX * WV), (g->nx + WT * WR - 1) / (WT * WR)), bg = box_grid(e, g->nx, g->ny);
@@ -940,14 +943,14 @@ int tm2d_run(const LensTM2D *g, const LensStepTable *tab, const LensEpi2D *ep, c
             if (epi2d_beyond_boxes(&e, n)) go([&] { tm2d_epi<<<grd, blk, 0, s>>>(*g, *tab, e, n); });
             else if (bg.x > 0) go([&] { box2d<<<bg, blk, 0, s>>>(*g, e); });
         }
-        return count ? LENS_OK : lens_cuda_status();
+        return dry ? LENS_OK : lens_cuda_status();
     }
     for (int n = n0; n < n0 + nsteps; ++n) {
         go([&] { tm2d_h<<<grd, blk, 0, s>>>(*g); });
         go([&] { tm2d_e<<<grd, blk, 0, s>>>(*g, *tab, n, d); });
         if (epi2d_active(&e, n)) go([&] { tm2d_epi<<<grd, blk, 0, s>>>(*g, *tab, e, n); });
     }
-    return count ? LENS_OK : lens_cuda_status();
+    return dry ? LENS_OK : lens_cuda_status();
 }
 
 }  // namespace
@@ -972,17 +975,27 @@ extern "C" int lens_tm2d_step_rows(const LensTM2D *g, const int *rowref, const L
     return tm2d_run(g, tab, ep, nullptr, n0, nsteps, stream, rowref);
 }
 
+extern "C" int lens_te2d_step_counted(const LensTE2D *g, const int *rowref, const LensStepTable *tab, const LensEpi2D *ep,
+                                      const LensDrive2D *drive, int n0, int nsteps, int *launches, void *stream) {
+    return te2d_run(g, tab, ep, drive, n0, nsteps, stream, rowref, launches);
+}
+
 extern "C" int lens_te2d_step_launches(const LensTE2D *g, const LensStepTable *tab, const LensEpi2D *ep,
                                        const LensDrive2D *drive, int n0, int nsteps) {
     int n = 0;
-    const int st = te2d_run(g, tab, ep, drive, n0, nsteps, nullptr, nullptr, &n);
+    const int st = te2d_run(g, tab, ep, drive, n0, nsteps, nullptr, nullptr, &n, true);
     return st == LENS_OK ? n : st;
+}
+
+extern "C" int lens_tm2d_step_counted(const LensTM2D *g, const int *rowref, const LensStepTable *tab, const LensEpi2D *ep,
+                                      const LensDrive2D *drive, int n0, int nsteps, int *launches, void *stream) {
+    return tm2d_run(g, tab, ep, drive, n0, nsteps, stream, rowref, launches);
 }
 
 extern "C" int lens_tm2d_step_launches(const LensTM2D *g, const LensStepTable *tab, const LensEpi2D *ep,
                                        const LensDrive2D *drive, int n0, int nsteps) {
     int n = 0;
-    const int st = tm2d_run(g, tab, ep, drive, n0, nsteps, nullptr, nullptr, &n);
+    const int st = tm2d_run(g, tab, ep, drive, n0, nsteps, nullptr, nullptr, &n, true);
     return st == LENS_OK ? n : st;
 }
 

@@ -242,18 +242,20 @@ class Grid2D:
                             _ptr(self.psi['hzx']), _ptr(self.psi['hzy']), _ptr(self.psi['exy']),
                             _ptr(self.psi['eyx']), pec4, s)
 
-        # scratch and error word of the resident launch (lens_te2d_resident), when the grid fits the chip;
-        # launches: kernel launches step() has made
-        self.launches = 0
-        need = (self.lib.lens_te2d_resident_bytes if self.pol == 's' else self.lib.lens_tm2d_resident_bytes)(
-            ctypes.byref(self.s))
+        lib, te = self.lib, self.pol == 's'
+        self._step = lib.lens_te2d_step_counted if te else lib.lens_tm2d_step_counted
+        self._resident = lib.lens_te2d_resident if te else lib.lens_tm2d_resident
+        self._rows = lib.lens_te2d_row_table if te else lib.lens_tm2d_row_table
+        self._made = ctypes.c_int(0)
+        # scratch and error word of the resident launch (lens_te2d_resident), when the grid fits the chip
+        need = (lib.lens_te2d_resident_bytes if te else lib.lens_tm2d_resident_bytes)(ctypes.byref(self.s))
         self.rs_scratch = torch.empty(need, dtype=torch.uint8, device=dev) if need else None
         self.rs_err = torch.zeros(1, dtype=torch.int32, device=dev) if need else None
         self.rs_stream = None       # stream of the last resident launch
         self.rs_plan = None         # rows, threads and bands of that launch; steps from which by sums, their most
         if need:
             plan = [ctypes.c_int() for _ in range(3)]
-            fn = self.lib.lens_te2d_resident_rows if self.pol == 's' else self.lib.lens_tm2d_resident_rows
+            fn = lib.lens_te2d_resident_rows if te else lib.lens_tm2d_resident_rows
             N.check(fn(ctypes.byref(self.s), 0, *map(ctypes.byref, plan)))
             self.rs_plan = tuple(v.value for v in plan)
             self.rs_steps = [resident_steps(self.pol, *self.rs_plan, q) for q in range(5)]
@@ -284,42 +286,43 @@ class Grid2D:
             if 0 < n < a.shape[0]:
                 a[:a.shape[0] - n].copy_(b[n:])
 
+    @property
+    def launches(self):
+        """Kernel launches that step() has made."""
+        return self._made.value
+
+    @launches.setter
+    def launches(self, n):
+        self._made.value = n
+
     def step(self, table, n0, nsteps, epi=None, stream=None, drive=None):
+        # one native call a span: a second, for the launch count, took 1.1 us of the 11.5 of a one-step call
+        n0, nsteps = int(n0), int(nsteps)
         e = ctypes.byref(epi.s) if epi is not None else None
-        if drive is None and self.rs_scratch is not None and nsteps >= RS_MIN_STEPS and (
-                nsteps >= self.rs_most or nsteps >= self.rs_steps[sums_a_step(epi.s, int(n0), int(nsteps)) if epi else 0]):
-            fn = self.lib.lens_te2d_resident if self.pol == 's' else self.lib.lens_tm2d_resident
-            on = stream if stream is not None else torch.cuda.current_stream()
-            st = fn(ctypes.byref(self.s), ctypes.byref(table.s), e, int(n0), int(nsteps), _ptr(self.rs_scratch),
-                    self.rs_scratch.numel(), _ptr(self.rs_err), _stream_ptr(on))
-            if st != N.ERR_SIZE:      # else: a call that only the steps below carry
-                self.launches += 1
-                self.rs_stream = on
-                return N.check(st)
-        te = self.pol == 's'
-        d = ctypes.byref(drive.s) if drive is not None else None
-        span = (ctypes.byref(table.s), e)
-        fn = self.lib.lens_te2d_step_launches if te else self.lib.lens_tm2d_step_launches
-        made = fn(ctypes.byref(self.s), *span, d, int(n0), int(nsteps))
-        N.check(min(0, made))
+        rows = None
         if drive is None:
-            fn = self.lib.lens_te2d_step_rows if te else self.lib.lens_tm2d_step_rows
-            rows = self._row_table(e, nsteps, stream)
-            N.check(fn(ctypes.byref(self.s), rows, *span, int(n0), int(nsteps), _stream_ptr(stream)))
-            made += 2 if rows is not None else 0
-        else:
-            fn = self.lib.lens_te2d_step_driven if te else self.lib.lens_tm2d_step_driven
-            N.check(fn(ctypes.byref(self.s), *span, d, int(n0), int(nsteps), _stream_ptr(stream)))
-        self.launches += made
+            if self.rs_scratch is not None and nsteps >= RS_MIN_STEPS and (
+                    nsteps >= self.rs_most or nsteps >= self.rs_steps[sums_a_step(epi.s, n0, nsteps) if epi else 0]):
+                on = stream if stream is not None else torch.cuda.current_stream()
+                st = self._resident(ctypes.byref(self.s), ctypes.byref(table.s), e, n0, nsteps, _ptr(self.rs_scratch),
+                                    self.rs_scratch.numel(), _ptr(self.rs_err), _stream_ptr(on))
+                if st != N.ERR_SIZE:      # else: a call that only the steps below carry
+                    self._made.value += 1
+                    self.rs_stream = on
+                    return N.check(st)
+            if self.rowref is not None:
+                rows = self._row_table(e, nsteps, stream)
+        d = ctypes.byref(drive.s) if drive is not None else None
+        N.check(self._step(ctypes.byref(self.s), rows, ctypes.byref(table.s), e, d, n0, nsteps, ctypes.byref(self._made),
+                           _stream_ptr(stream)))
+        if rows is not None:
+            self._made.value += 2
 
     def _row_table(self, e, nsteps, stream):
         """The table of repeated coefficient rows for a span of nsteps, from the coefficients as
-        they are now (they may be written between calls in any way); NULL where the span would
+        they are now (they may be written between calls in any way); None where the span would
         not gain by it."""
-        if self.rowref is None:
-            return None
-        fn = self.lib.lens_te2d_row_table if self.pol == 's' else self.lib.lens_tm2d_row_table
-        st = fn(ctypes.byref(self.s), e, int(nsteps), _ptr(self.rowref), _stream_ptr(stream))
+        st = self._rows(ctypes.byref(self.s), e, nsteps, _ptr(self.rowref), _stream_ptr(stream))
         if st == N.ERR_SIZE:
             return None
         N.check(st)

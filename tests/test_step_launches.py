@@ -51,3 +51,28 @@ def test_launches_of_a_step(pol, nx, ny, plain, box, window):
     assert _count(pol, nx, ny, _epi(box=True), ptr=20) == 10 * one           # so with arrays off 16 bytes
     assert _count(pol, nx, ny, n=0) == 0
     assert _count(pol, nx, ny, n0=95) == -1                                  # beyond the table: refused
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize('pol,nx,ny', [('s', 140, 96), ('p', 140, 96), ('p', 4000, 200), ('s', 9001, 513)])
+def test_grid_counts_what_its_spans_launch(pol, nx, ny):
+    """Grid2D.launches against the counting entry, over short spans and a driven one (no rows driven)."""
+    import torch
+    from lens_sensor_b200 import engine as E
+    from test_grid2d_resident import _grid as grid
+    g = grid(pol, nx, ny, True, 5)
+    fn = g.lib.lens_te2d_step_launches if pol == 's' else g.lib.lens_tm2d_step_launches
+    tab = E.StepTable(7, 4, g.dt, 2.2e15, 2.2e15, E.cw_envelope(3.5e14))
+    ep = E.Epi2D(g, boxes=[(2, nx // 3, 3, ny - 2)], dft=(8, 9))
+    drive = type('D', (), {'s': N.Drive2D()})()
+    for n, e, d in ((1, None, None), (3, ep, None), (2, ep, drive), (0, ep, None)):
+        want = fn(ctypes.byref(g.s), ctypes.byref(tab.s), ctypes.byref(e.s) if e else None,
+                  ctypes.byref(d.s) if d else None, 7, n)
+        was = g.launches
+        g.step(tab, 7, n, e, drive=d)
+        assert g.launches - was == want
+    was = g.launches
+    with pytest.raises(N.LensError):
+        g.step(tab, 7, 5, ep)
+    assert g.launches == was
+    torch.cuda.synchronize()
