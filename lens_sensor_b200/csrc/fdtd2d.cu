@@ -835,8 +835,10 @@ bool drive2d_ok(const LensDrive2D *d, const LensStepTable *tab, int nx) {
 // it in strips: us a step, one cell a thread / wide, TM 20.6 / 22.7 on 4000 x 128 cells and
 // 27.7 / 22.7 on 4000 x 200; TE with boxes 22.5 / 22.7 on 4000 x 256 and 26.5 / 24.0 on 4000 x
 // 300; TE inside its DFT windows, which the one-cell pass sums while it holds the field,
-// 34.9 / 39.3 on 4000 x 300 and 62.6 / 61.0 on 4000 x 500.
-constexpr double WIDE_TM = 0.7e6, WIDE_TE = 1.1e6, WIDE_TE_WINDOW = 1.9e6;  // cells
+// 34.9 / 39.3 on 4000 x 300 and 62.6 / 61.0 on 4000 x 500; TM inside them, whose sums are a third
+// launch either way, 33.0 / 39.1 on 5000 x 200, 38.3 / 42.2 on 6500 x 200, 38.9 / 38.8 on 3600 x 400
+// and, with Ex's sums, 58.9 / 55.2 on 4000 x 400 (wide H and one-cell E: 35.1, 40.0, 38.8).
+constexpr double WIDE_TM = 0.7e6, WIDE_TM_WINDOW = 1.4e6, WIDE_TE = 1.1e6, WIDE_TE_WINDOW = 1.9e6;  // cells
 
 bool wide_ok(const LensEpi2D &e, const LensDrive2D *dr, std::initializer_list<const void *> arrays) {
     if (dr || e.nsx > 0 || e.dft_raw || e.ex2) return false;
@@ -935,11 +937,17 @@ int tm2d_run(const LensTM2D *g, const LensStepTable *tab, const LensEpi2D *ep, c
     cudaStream_t s = static_cast<cudaStream_t>(stream);
     const Launch go{count, dry};
     const dim3 blk(BX, BY), grd((g->ny + BX - 1) / BX, (g->nx + BY - 1) / BY);
-    if ((double)g->nx * g->ny >= WIDE_TM && wide_ok(e, dr, {g->ex, g->ey, g->hz, g->ca_x, g->ca_y, g->da_x, g->da_y})) {
+    const double cells = (double)g->nx * g->ny;
+    if (cells >= WIDE_TM && wide_ok(e, dr, {g->ex, g->ey, g->hz, g->ca_x, g->ca_y, g->da_x, g->da_y})) {
         const dim3 wb(BX, WT), wg((g->ny + BX * WV - 1) / (BX * WV), (g->nx + WT * WR - 1) / (WT * WR)), bg = box_grid(e, g->nx, g->ny);
         for (int n = n0; n < n0 + nsteps; ++n) {
-            go([&] { tm2d_h_wide<<<wg, wb, 0, s>>>(*g); });
-            go([&] { tm2d_e_wide<<<wg, wb, 0, s>>>(*g, rowref, *tab, n); });
+            if (cells < WIDE_TM_WINDOW && epi2d_beyond_boxes(&e, n)) {
+                go([&] { tm2d_h<<<grd, blk, 0, s>>>(*g); });
+                go([&] { tm2d_e<<<grd, blk, 0, s>>>(*g, *tab, n, d); });
+            } else {
+                go([&] { tm2d_h_wide<<<wg, wb, 0, s>>>(*g); });
+                go([&] { tm2d_e_wide<<<wg, wb, 0, s>>>(*g, rowref, *tab, n); });
+            }
             if (epi2d_beyond_boxes(&e, n)) go([&] { tm2d_epi<<<grd, blk, 0, s>>>(*g, *tab, e, n); });
             else if (bg.x > 0) go([&] { box2d<<<bg, blk, 0, s>>>(*g, e); });
         }

@@ -132,3 +132,20 @@ def test_wide_passes_without_a_table(case):
     _same(a, b)
     for q in ('dft', 'prev', 'iavg'):
         assert torch.equal(getattr(ea, q), getattr(eb, q)), q
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize('nx,ny', [(6900, 101), (5000, 200), (3501, 399), (3499, 401)])
+@pytest.mark.parametrize('lossy', [True, False])
+def test_tm_spans_into_their_windows(nx, ny, lossy):
+    """TM grids on either side of the size from which the wide passes run inside the windows too."""
+    import torch
+    a, b = (_grid('p', nx, ny, lossy, 9) for _ in range(2))
+    tab = _tab(a, 9)
+    ea, eb = _epi(a, 9, True), _epi(b, 9, True)
+    assert a.lib.lens_tm2d_step_rows(ctypes.byref(a.s), None, ctypes.byref(tab.s), ctypes.byref(ea.s), 7, 9, None) == 0
+    _one_cell(b, tab, 7, 9, eb)
+    torch.cuda.synchronize()
+    _same(a, b)
+    for q in ('dft', 'dft_ex', 'prev', 'iavg'):
+        assert torch.equal(getattr(ea, q), getattr(eb, q)), q
