@@ -1480,8 +1480,9 @@ int make_chunks(const LensGrid3D *g, int target, int *x, int *strip) {
         strip[n] = s;
         x[++n] = b;
     };
+    auto strips_of = [&](int a, int b) { return std::min((b - a + target - 1) / target, 16); };
     auto add_strip = [&](int a, int b) {
-        const int np = std::min((b - a + target - 1) / target, 16);
+        const int np = strips_of(a, b);
         for (int q = 0; q < np; ++q) add(a + (int)((long)(b - a) * q / np), a + (int)((long)(b - a) * (q + 1) / np), 1);
     };
     if (lo > 0) add_strip(0, lo);
@@ -1489,7 +1490,7 @@ int make_chunks(const LensGrid3D *g, int target, int *x, int *strip) {
     if (mid > 0) {
         int pieces = (mid + target / 2) / target;
         if (pieces < 1) pieces = 1;
-        if (pieces > MAXCH - 34) pieces = MAXCH - 34;
+        pieces = std::min(pieces, MAXCH - n - strips_of(hi, nx));  // at least MAXCH - 32
         for (int q = 0; q < pieces; ++q)
             add(lo + (int)((long)mid * q / pieces), lo + (int)((long)mid * (q + 1) / pieces), 0);
     }
@@ -1515,7 +1516,9 @@ void lean_range(int count, F is_strip, int &l0, int &l1) {
 // warm-up plane and start), a launch as long as its longest CTA, or its whole work over
 // the slots and a share of one lean chunk for the last CTAs' tail.  With chunks chosen for
 // whole waves of equal CTAs alone, at least 12 planes long, 64 x 48 x 40 cells took 51 us a
-// step (the CPML tiles' 12 planes one after another) and 200 x 100 x 120 took 97.
+// step (the CPML tiles' 12 planes one after another) and 200 x 100 x 120 took 97.  With the
+// tail charged to CTAs that are all resident too, 1000 x 33 x 40 took 104 us for 84 and 300 x 33 x
+// 65 53 for 41; with at most 62 lean chunks, 1200 x 30 x 30 68.5 for 54.9.
 constexpr int PLANE_COST[4] = {10, 14, 19, 23};  // tenths of a lean plane (1.6 us), by axes
 Work make_work(const LensGrid3D *g, int slots) {
     Work wk{};
@@ -1548,7 +1551,8 @@ Work make_work(const LensGrid3D *g, int slots) {
                 longest = std::max(longest, w);
             }
         }
-        const double cost = std::max(longest, total / (slots > 0 ? slots : 1) + 0.35 * lean);
+        double cost = std::max(longest, total / (slots > 0 ? slots : 1) + 0.35 * lean);
+        if ((long)ntz * nty * nc <= slots) cost = longest;  // every CTA resident at once: no tail
         if (cost < best - 1e-9) {
             best = cost;
             target = t;

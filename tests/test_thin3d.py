@@ -1,5 +1,6 @@
-"""3D grids whose x absorbers meet (every x plane a strip plane): the fused pass against the
-two streaming passes, and nothing written behind the last plane."""
+"""3D grids at the ends of the fused pass's x chunks, against the two streaming passes: grids
+whose x absorbers meet (every x plane a strip plane; nothing written behind the last), and long
+thin ones with as many chunks as there may be or as the chip holds at once."""
 import numpy as np
 import pytest
 
@@ -21,8 +22,15 @@ def _grid(dims, lossy, fused):
     for q in g.FIELDS:
         v = g.view(q)
         v.copy_(torch.from_numpy((rng.standard_normal(tuple(v.shape)) / (1 if q[0] == 'e' else 377)).astype(np.float32)))
-    assert g.s.ax.e.lo == nx and g.s.ax.h.lo == nx - 1
     return g
+
+
+def _close(a, b):
+    for names in ('ex ey ez', 'hx hy hz'):
+        v = [[g.view(q).double() for q in names.split()] for g in (a, b)]
+        norm = float(sum((t ** 2).sum() for t in v[1])) ** 0.5
+        for x, y in zip(*v):
+            assert float((x - y).norm()) <= TOL * norm
 
 
 @pytest.mark.gpu
@@ -32,6 +40,7 @@ def test_x_all_absorber(dims, lossy):
     from lens_sensor_b200 import engine as E
     nx, ny, nz = dims
     a, b = _grid(dims, lossy, True), _grid(dims, lossy, False)
+    assert a.s.ax.e.lo == nx and a.s.ax.h.lo == nx - 1
     # the fused grid's two buffers with one more plane each, which has to stay as it is
     big = []
     for k in range(2):
@@ -47,8 +56,19 @@ def test_x_all_absorber(dims, lossy):
     torch.cuda.synchronize()
     a.check_flag()
     assert all(bool((t[nx] == 7.0).all()) for t in big)
-    for names in ('ex ey ez', 'hx hy hz'):
-        v = [[g.view(q).double() for q in names.split()] for g in (a, b)]
-        norm = float(sum((t ** 2).sum() for t in v[1])) ** 0.5
-        for x, y in zip(*v):
-            assert float((x - y).norm()) <= TOL * norm
+    _close(a, b)
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize('dims,lossy', [((1200, 30, 30), False), ((1000, 33, 40), True), ((301, 33, 65), False), ((2500, 8, 20), True),
+                                        ((601, 65, 97), False)])
+def test_long_and_thin(dims, lossy):
+    import torch
+    from lens_sensor_b200 import engine as E
+    a, b = _grid(dims, lossy, True), _grid(dims, lossy, False)
+    tab = E.StepTable(0, 9, a.dt, 2.2e15, 2.2e15, E.cw_envelope(3.5e14))
+    for g in (a, b):
+        g.step(tab, 0, 9)
+    torch.cuda.synchronize()
+    a.check_flag()
+    _close(a, b)
