@@ -16,6 +16,7 @@
 // then the Huygens source (vcsel.py:151-156) and the PEC termination
 // (boundaries.py:207-215, 260-268) in the reference order (inject, then PEC).
 #include <algorithm>
+#include <cmath>
 #include <initializer_list>
 
 #include "lens_common.cuh"
@@ -753,23 +754,6 @@ __global__ void __launch_bounds__(BX *BY) box2d(const G g, const LensEpi2D ep) {
     }
 }
 
-// Epilogue of the new Ez after a wide E pass.
-__global__ void __launch_bounds__(BX *BY)
-    te2d_epi(const LensTE2D g, const LensStepTable tab, const LensEpi2D ep, int n) {
-    const int j = blockIdx.x * BX + threadIdx.x, i = blockIdx.y * BY + threadIdx.y;
-    const bool valid = i < g.nx && j < g.ny;
-    const int P = g.pitch;
-    const size_t o = (size_t)i * P + j;
-    float ez = 0.f;
-    if (valid) {
-        ez = g.ez[o];
-        if (ep.nplane > 0 && in_window(ep, n))
-            for (int p = 0; p < ep.nplane; ++p)
-                if (i == ep.plane[p]) plane_node(ep, tab, n, p, P, j, ez, 0.5f * (g.hy[o - P] + g.hy[o]));
-    }
-    epilogue_node(ep, tab, n, i, j, valid, o, ez, __fmul_rn(ez, ez), 0.f);
-}
-
 // Does the epilogue do more at step n than sum its boxes?
 bool epi2d_beyond_boxes(const LensEpi2D *ep, int n) {
     if (!ep) return false;
@@ -830,15 +814,47 @@ bool drive2d_ok(const LensDrive2D *d, const LensStepTable *tab, int nx) {
 }
 
 // The wide passes carry every plain step whose arrays start on 16-byte boundaries; the
-// stitch drive, the stitch sums and the pulse planes stay with one cell a thread.  A small
-// grid's passes last as long as one warp, and a wide one does eight times the work, half of
-// it in strips: us a step, one cell a thread / wide, TM 20.6 / 22.7 on 4000 x 128 cells and
-// 27.7 / 22.7 on 4000 x 200; TE with boxes 22.5 / 22.7 on 4000 x 256 and 26.5 / 24.0 on 4000 x
-// 300; TE inside its DFT windows, which the one-cell pass sums while it holds the field,
-// 34.9 / 39.3 on 4000 x 300 and 62.6 / 61.0 on 4000 x 500; TM inside them, whose sums are a third
-// launch either way, 33.0 / 39.1 on 5000 x 200, 38.3 / 42.2 on 6500 x 200, 38.9 / 38.8 on 3600 x 400
-// and, with Ex's sums, 58.9 / 55.2 on 4000 x 400 (wide H and one-cell E: 35.1, 40.0, 38.8).
-constexpr double WIDE_TM = 0.7e6, WIDE_TM_WINDOW = 1.4e6, WIDE_TE = 1.1e6, WIDE_TE_WINDOW = 1.9e6;  // cells
+// stitch drive, the stitch sums and the pulse planes stay with one cell a thread.  They take
+// 1024 cells a block, whole column blocks, and their warps at a y face run with tests: a
+// grid has to be large, and more so a narrow one, whose last block is mostly idle.  us a
+// step, one cell a thread / wide: TM 26.9 / 26.6 on 4251 x 400, 31.0 / 31.0 on 8595 x 256, 45.3 /
+// 46.7 on 16923 x 130, 67.9 / 63.1 on 23075 x 130, 106.9 / 118.9 on 78123 x 64, 119 / 240 on 166667
+// x 30; TE 22.6 / 25.1 on 5003 x 200 and 26.9 / 26.8 on 6499 x 200, 53.5 / 61.5 on 46875 x 64, 107 /
+// 102 on 78123 x 64, 121 / 207 on 166667 x 30.  (By cells alone, from 0.7 M TM and 1.1 M TE, steps
+// took up to 1.5 and 1.9 times the one-cell passes': 12000 x 64 TM, 40000 x 30 TE.)
+bool wide_tm(double cells, int ny) {
+    const int cb = (ny + BX * WV - 1) / (BX * WV);
+    const double pad = (double)cb * BX * WV / ny;
+    if (cb > 3) return cells >= 1.5e6;
+    return pad <= 2.0 && cells >= 2.2e6 * std::sqrt(pad) * (cb == 1 && pad > 1.5 ? 2.3 : 1.0);
+}
+
+bool wide_te(double cells, int ny) {
+    const int cb = (ny + BX * WV - 1) / (BX * WV);
+    const double pad = (double)cb * BX * WV / ny;
+    return pad <= 2.0 && cells >= (cb == 1 && pad > 1.5 ? 5e6 : 1.1e6);
+}
+
+// TE grids whose wide passes gain whatever a step's epilogue.  Below, the one-cell E pass, which
+// sums small boxes while it holds the field (32 us a million nodes), is faster than the wide passes and
+// a launch of the boxes (4 us): 26.1 / 30.3 us a step on 5075 x 256 with boxes of 4000 nodes, 31.0 /
+// 30.9 on 6643 x 256, 26.9 / 26.8 on 4331 x 300; and a step with sums keeps its H pass too: 41.2 / 43.2
+// on 5075 x 256, 51.7 / 52.0 on 6643 x 256, 53.5 / 53.5 on 4251 x 400.
+bool firm_te(double cells, int ny) { return cells >= (ny > 2 * BX * WV ? 1.3e6 : 1.8e6); }
+
+// A TE step with sums has a wide H and the one-cell E pass, which adds to them while it holds the
+// field: one cell / wide with the sums in a launch of their own / this: 79.6 / 88.1 / 78.2 us a step
+// on 11003 x 200, 353 / 332 / 313 on 14283 x 700.
+// TM's sums are a launch of their own either way, and its boxes have one (box2d, not the epilogue
+// over the whole grid) from TM_BOX cells, whatever the passes: 33.2 -> 24.7 us a step on 5387 x 130.
+constexpr double TM_BOX = 0.7e6;
+
+double box_nodes(const LensEpi2D &e) {
+    double nodes = 0.0;
+    for (int b = 0; b < e.nbox; ++b)
+        nodes += (double)std::max(0, e.box[b][1] - e.box[b][0]) * std::max(0, e.box[b][3] - e.box[b][2]);
+    return nodes;
+}
 
 bool wide_ok(const LensEpi2D &e, const LensDrive2D *dr, std::initializer_list<const void *> arrays) {
     if (dr || e.nsx > 0 || e.dft_raw || e.ex2) return false;
@@ -903,17 +919,20 @@ int te2d_run(const LensTE2D *g, const LensStepTable *tab, const LensEpi2D *ep, c
     const Launch go{count, dry};
     const dim3 blk(BX, BY), grd((g->ny + BX - 1) / BX, (g->nx + BY - 1) / BY);
     const double cells = (double)g->nx * g->ny;
-    if (cells >= WIDE_TE && wide_ok(e, dr, {g->ez, g->hx, g->hy, g->ce_e, g->ce_h})) {
+    if (wide_te(cells, g->ny) && wide_ok(e, dr, {g->ez, g->hx, g->hy, g->ce_e, g->ce_h})) {
         const dim3 wb(BX, WT), wg((g->ny + BX * WV - 1) / (BX * WV), (g->nx + WT * WR - 1) / (WT * WR)), bg = box_grid(e, g->nx, g->ny);
+        const double nodes = box_nodes(e);
+        const bool firm = firm_te(cells, g->ny), wide = firm || nodes == 0.0 || nodes >= 0.12e6;
         for (int n = n0; n < n0 + nsteps; ++n) {
-            go([&] { te2d_h_wide<<<wg, wb, 0, s>>>(*g); });
-            if (cells < WIDE_TE_WINDOW && epi2d_beyond_boxes(&e, n)) {
+            const bool sums = epi2d_beyond_boxes(&e, n);
+            if (sums ? firm : wide) go([&] { te2d_h_wide<<<wg, wb, 0, s>>>(*g); });
+            else go([&] { te2d_h<<<grd, blk, 0, s>>>(*g); });
+            if (sums || !wide) {
                 go([&] { te2d_e<<<grd, blk, 0, s>>>(*g, *tab, e, n, d); });
                 continue;
             }
             go([&] { te2d_e_wide<<<wg, wb, 0, s>>>(*g, rowref, *tab, n); });
-            if (epi2d_beyond_boxes(&e, n)) go([&] { te2d_epi<<<grd, blk, 0, s>>>(*g, *tab, e, n); });
-            else if (bg.x > 0) go([&] { box2d<<<bg, blk, 0, s>>>(*g, e); });
+            if (bg.x > 0) go([&] { box2d<<<bg, blk, 0, s>>>(*g, e); });
         }
         return dry ? LENS_OK : lens_cuda_status();
     }
@@ -938,15 +957,16 @@ int tm2d_run(const LensTM2D *g, const LensStepTable *tab, const LensEpi2D *ep, c
     const Launch go{count, dry};
     const dim3 blk(BX, BY), grd((g->ny + BX - 1) / BX, (g->nx + BY - 1) / BY);
     const double cells = (double)g->nx * g->ny;
-    if (cells >= WIDE_TM && wide_ok(e, dr, {g->ex, g->ey, g->hz, g->ca_x, g->ca_y, g->da_x, g->da_y})) {
+    const bool ok = wide_ok(e, dr, {g->ex, g->ey, g->hz, g->ca_x, g->ca_y, g->da_x, g->da_y}), wide = ok && wide_tm(cells, g->ny);
+    if (wide || (ok && cells >= TM_BOX)) {
         const dim3 wb(BX, WT), wg((g->ny + BX * WV - 1) / (BX * WV), (g->nx + WT * WR - 1) / (WT * WR)), bg = box_grid(e, g->nx, g->ny);
         for (int n = n0; n < n0 + nsteps; ++n) {
-            if (cells < WIDE_TM_WINDOW && epi2d_beyond_boxes(&e, n)) {
-                go([&] { tm2d_h<<<grd, blk, 0, s>>>(*g); });
-                go([&] { tm2d_e<<<grd, blk, 0, s>>>(*g, *tab, n, d); });
-            } else {
+            if (wide) {
                 go([&] { tm2d_h_wide<<<wg, wb, 0, s>>>(*g); });
                 go([&] { tm2d_e_wide<<<wg, wb, 0, s>>>(*g, rowref, *tab, n); });
+            } else {
+                go([&] { tm2d_h<<<grd, blk, 0, s>>>(*g); });
+                go([&] { tm2d_e<<<grd, blk, 0, s>>>(*g, *tab, n, d); });
             }
             if (epi2d_beyond_boxes(&e, n)) go([&] { tm2d_epi<<<grd, blk, 0, s>>>(*g, *tab, e, n); });
             else if (bg.x > 0) go([&] { box2d<<<bg, blk, 0, s>>>(*g, e); });
@@ -1010,7 +1030,7 @@ extern "C" int lens_tm2d_step_launches(const LensTM2D *g, const LensStepTable *t
 extern "C" int lens_te2d_row_table(const LensTE2D *g, const LensEpi2D *ep, int nsteps, int *rowref, void *stream) {
     if (!rowref) return LENS_ERR_ARG;
     if (!grid2d_ok(g) || !g->ce_e || !g->ce_h || !row_table_pays(g->nx, g->pitch, 5, nsteps) ||
-        (double)g->nx * g->ny < WIDE_TE || !wide_ok(ep ? *ep : empty_epi(), nullptr, {g->ez, g->hx, g->hy, g->ce_e, g->ce_h}))
+        !wide_te((double)g->nx * g->ny, g->ny) || !wide_ok(ep ? *ep : empty_epi(), nullptr, {g->ez, g->hx, g->hy, g->ce_e, g->ce_h}))
         return LENS_ERR_SIZE;
     return row_table(RowArrays{{g->ce_e, g->ce_h}, {g->nx, g->nx}, 2}, g->nx, g->ny, g->pitch, rowref, stream);
 }
@@ -1018,7 +1038,7 @@ extern "C" int lens_te2d_row_table(const LensTE2D *g, const LensEpi2D *ep, int n
 extern "C" int lens_tm2d_row_table(const LensTM2D *g, const LensEpi2D *ep, int nsteps, int *rowref, void *stream) {
     if (!rowref) return LENS_ERR_ARG;
     if (!grid2d_ok(g) || !g->ca_x || !g->ca_y || (!g->da_x) != (!g->da_y) ||
-        !row_table_pays(g->nx, g->pitch, g->da_x ? 7 : 5, nsteps) || (double)g->nx * g->ny < WIDE_TM ||
+        !row_table_pays(g->nx, g->pitch, g->da_x ? 7 : 5, nsteps) || !wide_tm((double)g->nx * g->ny, g->ny) ||
         !wide_ok(ep ? *ep : empty_epi(), nullptr, {g->ex, g->ey, g->hz, g->ca_x, g->ca_y, g->da_x, g->da_y}))
         return LENS_ERR_SIZE;
     return row_table(RowArrays{{g->ca_x, g->ca_y, g->da_x, g->da_y}, {g->nx - 1, g->nx, g->nx - 1, g->nx}, g->da_x ? 4 : 2},

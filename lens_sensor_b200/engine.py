@@ -125,7 +125,7 @@ def sums_a_step(e, n0, nsteps):
     w = met(e.dft_n0, e.dft_n1)
     k = (w if e.dft else 0) + (w if e.dft_ex else 0) + (met(e.prev_n0, e.prev_n1) if e.dft_prev else 0) + \
         (met(e.iavg_n0, n0 + nsteps) if e.iavg else 0)
-    return (2 * k + nsteps) // (2 * nsteps)
+    return (2 * k + nsteps) // max(2 * nsteps, 1)
 
 
 class _Axis:
@@ -313,7 +313,8 @@ class Grid2D:
                     self._made.value += 1
                     self.rs_stream = on
                     return N.check(st)
-            if self.rowref is not None:
+            # (TE steps with sums read every row: their E pass is the one-cell one)
+            if self.rowref is not None and not (epi is not None and self.pol == 's' and sums_a_step(epi.s, n0, nsteps)):
                 rows = self._row_table(e, nsteps, stream)
         d = ctypes.byref(drive.s) if drive is not None else None
         N.check(self._step(ctypes.byref(self.s), rows, ctypes.byref(table.s), e, d, n0, nsteps, ctypes.byref(self._made),

@@ -8,7 +8,7 @@ import pytest
 from lens_sensor_b200 import _native as N
 from test_grid2d_resident import FIELDS, WIDE, _epi, _grid
 
-SIZES = [('s', 9001, 513, False), ('s', 170001, 31, False), ('p', 7003, 449, True), ('p', 9100, 513, False), ('s', 40001, 100, False)]  # from the table's least size
+SIZES = [('s', 9001, 513, False), ('s', 90001, 65, False), ('p', 7003, 449, True), ('p', 9100, 513, False), ('s', 40001, 100, False)]  # from the table's least size
 
 
 def _coef(g):
@@ -149,3 +149,34 @@ def test_tm_spans_into_their_windows(nx, ny, lossy):
     _same(a, b)
     for q in ('dft', 'dft_ex', 'prev', 'iavg'):
         assert torch.equal(getattr(ea, q), getattr(eb, q)), q
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize('pol,nx,ny', [('s', 20001, 60), ('s', 39063, 128), ('s', 8999, 129), ('s', 4297, 256), ('s', 5061, 257),
+                                       ('s', 7039, 256), ('s', 80001, 64), ('p', 12001, 64), ('p', 25001, 129), ('p', 17001, 130),
+                                       ('p', 3901, 385), ('p', 8601, 256)])
+@pytest.mark.parametrize('small', [True, False])
+def test_either_side_of_the_wide_sizes(pol, nx, ny, small):
+    """Spans of a plain step, steps with boxes, and steps with sums, by grid and box size."""
+    import torch
+    from lens_sensor_b200 import engine as E
+    out = []
+    for k in range(2):
+        g = _grid(pol, nx, ny, pol == 'p' and small, 9)
+        tab = _tab(g, 6)
+        ep = E.Epi2D(g, boxes=[(5, 12, 3, ny - 2)] if small else [(5, nx // 2, 0, ny)], dft=(10, 12), dft_ex=pol == 'p')
+        for n, e in ((7, None), (8, ep)):
+            m = 1 if e is None else 5
+            if k:
+                fn = g.lib.lens_te2d_step_driven if pol == 's' else g.lib.lens_tm2d_step_driven
+                assert fn(ctypes.byref(g.s), ctypes.byref(tab.s), ctypes.byref(e.s) if e else None, ctypes.byref(N.Drive2D()),
+                          n, m, None) == 0
+            else:
+                fn = g.lib.lens_te2d_step if pol == 's' else g.lib.lens_tm2d_step
+                assert fn(ctypes.byref(g.s), ctypes.byref(tab.s), ctypes.byref(e.s) if e else None, n, m, None) == 0
+        torch.cuda.synchronize()
+        out.append((g, ep))
+    (a, ea), (b, eb) = out
+    _same(a, b)
+    assert torch.equal(ea.dft, eb.dft)
+    assert float((ea.box_acc - eb.box_acc).abs().max()) <= 1e-12 * float(eb.box_acc.abs().max())
