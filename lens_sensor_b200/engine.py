@@ -87,18 +87,19 @@ RS_MIN_STEPS = 4
 # has 168 (a CTA of more than 8 warps, or several on an SM), from 16 where it has 255.  Every
 # sum a step then costs more in the resident launch than in the passes.  By the sums a step runs
 # (DFT, TM Ex, comparison window, average), TE and TM; us a call, resident / step by step, on
-# either side of a line: TE 2400 x 513 with 3 sums 467 / 445 at 12 steps and 852 / 880 at 24, TE
-# 7000 x 90 with 2 275 / 254 and 471 / 506 at the same, TE 5000 x 180 with 1 113 / 99 at 4 and 120 /
-# 121 at 5.  TM, resident over step by step: 2400 x 448 with 4 sums 1.06 at 7 steps and 0.90 at 14,
-# 2700 x 400 with 4 1.06 at 11 and 0.91 at 44, 5000 x 200 with 4 1.03 at 6 and 0.91 at 12; 2000 x 513
-# with 4 1.08 at 20 and 1.00 at 80; the TM forms marked NEVER lose at any length: 2400 x 513 with 4
-# sums 1.1 to 1.3 at 64 to 256, 18 rows of 90 columns, 256 threads a CTA, with 3 1.04 at 64.
+# either side of a line: TE 2400 x 513 with 3 sums 724 / 660 at 20 steps and 2631 / 2629 at 80, 2000 x
+# 513 with 3 381 / 322 at 12 and 678 / 644 at 24, 8000 x 80 with 3 290 / 273 and 513 / 545 at the same.
+# TM, resident over step by step: 2400 x 513 without sums 1.08 at 6 and 0.84 at 12, 2400 x 448 with 4
+# 1.06 at 7 and 0.90 at 14, 2700 x 400 with 4 1.06 at 11 and 0.91 at 44, 5000 x 200 with 4 1.03 at 6
+# and 0.91 at 12, 2000 x 513 with 4 1.08 at 20 and 1.00 at 80; the TM forms marked NEVER lose at any
+# length: 2400 x 513 with 4 1.1 to 1.3 at 64 to 256, 18 rows of 90 columns, 256 threads a CTA, with 3
+# 1.04 at 64.
 NEVER = 1 << 30
 RS_SPILL_STEPS = [  # crowded (168 registers or several CTAs an SM), least rows, steps TE, steps TM
-    (True, 18, (5, 6, 12, 20), (6, 8, 32, 64, NEVER)),
-    (True, 16, (5, 6, 10, 12), (5, 5, 10, 12, 20)),
-    (True, 10, (4, 5, 7, 8), (4, 4, 5, 6, 8)),
-    (False, 20, (5, 6, 10, 14), (5, 4, 7, 10, 20)),
+    (True, 18, (5, 6, 12, 60), (7, 8, 32, 64, NEVER)),
+    (True, 16, (5, 6, 10, 24), (5, 5, 10, 12, 20)),
+    (True, 10, (4, 5, 7, 10), (4, 4, 5, 6, 8)),
+    (False, 20, (5, 6, 10, 16), (5, 4, 7, 10, 20)),
     (False, 16, (4, 5, 6, 10), (4, 4, 5, 6, 9))]
 
 

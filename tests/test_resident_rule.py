@@ -33,7 +33,7 @@ def test_steps_rise_with_rows_and_sums():
 
 @pytest.mark.gpu
 @pytest.mark.parametrize('pol,steps,window,launches', [
-    ('p', 24, True, 72), ('p', 24, False, 1), ('p', 4, False, 8), ('s', 12, True, 24), ('s', 20, True, 1)])
+    ('p', 24, True, 72), ('p', 24, False, 1), ('p', 4, False, 8), ('s', 12, True, 24), ('s', 60, True, 1)])
 def test_spans_of_a_full_chip(pol, steps, window, launches):
     """2400 x 513 cells, bands of 18 rows: inside its windows step by step (TM at any length)."""
     import torch
