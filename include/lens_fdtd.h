@@ -158,10 +158,10 @@ int lens_tm2d_step_rows(const LensTM2D *g, const int *rowref, const LensStepTabl
  * array, read from the arrays when the stream reaches the call.  The table holds for the
  * steps enqueued behind it until the coefficients are written again, so a caller forms it
  * anew before each span.  rowref: nx device ints.  LENS_ERR_SIZE, with nothing enqueued:
- * a span of nsteps on this grid with this epilogue (may be NULL) does not gain by it;
+ * the span [n0, n0 + nsteps) on this grid with this epilogue (may be NULL) does not gain by it;
  * step it with a NULL rowref.                                                 */
-int lens_te2d_row_table(const LensTE2D *g, const LensEpi2D *ep, int nsteps, int *rowref, void *stream);
-int lens_tm2d_row_table(const LensTM2D *g, const LensEpi2D *ep, int nsteps, int *rowref, void *stream);
+int lens_te2d_row_table(const LensTE2D *g, const LensEpi2D *ep, int n0, int nsteps, int *rowref, void *stream);
+int lens_tm2d_row_table(const LensTM2D *g, const LensEpi2D *ep, int n0, int nsteps, int *rowref, void *stream);
 
 /* Stitch-window drive of a 2D grid (fdtd2d_core.py:1439-1440, 1462-1463): after
  * each E update, before the PEC termination, the first nplanes x-rows of the

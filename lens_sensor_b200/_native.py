@@ -144,8 +144,8 @@ SIGNATURES = {
                                        c_int, POINTER(c_int), c_void_p]),
     'lens_te2d_step_launches': (c_int, [POINTER(TE2D), POINTER(StepTable), POINTER(Epi2D), POINTER(Drive2D), c_int, c_int]),
     'lens_tm2d_step_launches': (c_int, [POINTER(TM2D), POINTER(StepTable), POINTER(Epi2D), POINTER(Drive2D), c_int, c_int]),
-    'lens_te2d_row_table': (c_int, [POINTER(TE2D), POINTER(Epi2D), c_int, c_void_p, c_void_p]),
-    'lens_tm2d_row_table': (c_int, [POINTER(TM2D), POINTER(Epi2D), c_int, c_void_p, c_void_p]),
+    'lens_te2d_row_table': (c_int, [POINTER(TE2D), POINTER(Epi2D), c_int, c_int, c_void_p, c_void_p]),
+    'lens_tm2d_row_table': (c_int, [POINTER(TM2D), POINTER(Epi2D), c_int, c_int, c_void_p, c_void_p]),
     'lens_te2d_step_driven': (c_int, [POINTER(TE2D), POINTER(StepTable), POINTER(Epi2D), POINTER(Drive2D), c_int,
                                       c_int, c_void_p]),
     'lens_tm2d_step_driven': (c_int, [POINTER(TM2D), POINTER(StepTable), POINTER(Epi2D), POINTER(Drive2D), c_int,

@@ -829,6 +829,22 @@ bool wide_tm(double cells, int ny) {
     return pad <= 2.0 && cells >= 2.2e6 * std::sqrt(pad) * (cb == 1 && pad > 1.5 ? 2.3 : 1.0);
 }
 
+// TM inside its windows, whose sums are a launch of their own either way: the one-cell passes stay in
+// front while fields, coefficients and sums lie in the L2.  us a step, one cell a thread / wide: 44.0 /
+// 47.4 on 7500 x 200 with the DFT's sums (74 MB), 77.9 / 76.5 with every sum and loss (134 MB); 67.8 /
+// 63.5 on 14800 x 100 with the DFTs' and loss (113 MB); 3600 x 400 38.8 / 38.9 (66 MB) and 45.2 / 43.8 (78).
+bool wide_tm_sums(double cells, int ny, double bytes) {
+    const int cb = (ny + BX * WV - 1) / (BX * WV);
+    return wide_tm(cells, ny) || (cells >= 1.4e6 && 2.0 * cb * BX * WV <= 3.0 * ny && bytes >= (cb > 2 ? 70e6 : 110e6));
+}
+
+// Bytes a node of the sums that step n adds to.
+int sum_bytes(const LensEpi2D &e, int n) {
+    const bool win = n >= e.dft_n0 && n < e.dft_n1;
+    return (win && e.dft ? 16 : 0) + (win && e.dft_ex ? 16 : 0) + (e.dft_prev && n >= e.prev_n0 && n < e.prev_n1 ? 16 : 0) +
+           (e.iavg && n >= e.iavg_n0 ? 4 : 0);
+}
+
 bool wide_te(double cells, int ny) {
     const int cb = (ny + BX * WV - 1) / (BX * WV);
     const double pad = (double)cb * BX * WV / ny;
@@ -840,7 +856,7 @@ bool wide_te(double cells, int ny) {
 // a launch of the boxes (4 us): 26.1 / 30.3 us a step on 5075 x 256 with boxes of 4000 nodes, 31.0 /
 // 30.9 on 6643 x 256, 26.9 / 26.8 on 4331 x 300; and a step with sums keeps its H pass too: 41.2 / 43.2
 // on 5075 x 256, 51.7 / 52.0 on 6643 x 256, 53.5 / 53.5 on 4251 x 400.
-bool firm_te(double cells, int ny) { return cells >= (ny > 2 * BX * WV ? 1.3e6 : 1.8e6); }
+bool firm_te(double cells, int ny) { return cells >= (ny > 2 * BX * WV ? 1.2e6 : 1.8e6); }
 
 // A TE step with sums has a wide H and the one-cell E pass, which adds to them while it holds the
 // field: one cell / wide with the sums in a launch of their own / this: 79.6 / 88.1 / 78.2 us a step
@@ -864,18 +880,36 @@ bool wide_ok(const LensEpi2D &e, const LensDrive2D *dr, std::initializer_list<co
 }
 
 // A span forms a row table where the coefficients come from memory, not from the L2 (126
-// MB): by the bytes of fields and coefficients.  us a step without / with the table: TM 1600 x
+// MB): by the bytes of fields, coefficients and the sums that TM's steps add to (TE's read every
+// row, in their one-cell E pass).  us a step without / with the table: TM 1600 x
 // 480 to 4000 x 448 cells (50 MB) the same within 0.5 %, 4000 x 700 (79 MB) 36.1 / 33.3, 16000 x
 // 200 (100 MB) 61.9 / 51.3, 8000 x 700 (158 MB) 69.9 / 49.9, 16000 x 700 (315 MB) 122.8 / 105.7;
 // TE 16000 x 200 (72 MB) 47.0 / 46.6, 8000 x 700 (113 MB) 51.9 / 43.1, 16000 x 700 (225 MB) 102.4
-// / 95.0.  Forming it takes 19 to 52 us, two to four steps' gain; a grid without repeated
+// / 95.0; TM inside its windows, every sum and loss, one cell a thread without: 3600 x 400 (120 MB)
+// 64.0 / 57.5, 14800 x 100 80.1 / 75.1, 9000 x 130 63.0 / 58.9.  Forming it takes 19 to 52 us, two to four steps' gain; a grid without repeated
 // rows loses that, 5 % of the shortest span that forms one.  (Formed once with the grid and
 // kept, the table went stale when the coefficients were written past its check.)
 constexpr double ROW_BYTES = 90e6;
 constexpr int ROW_STEPS = 8;
 
-bool row_table_pays(int nx, int P, int arrays, int nsteps) {
-    return nsteps >= ROW_STEPS && 4.0 * nx * P * arrays >= ROW_BYTES;
+bool row_table_pays(int nx, int P, int arrays, double sums, int nsteps) {
+    return nsteps >= ROW_STEPS && (4.0 * arrays + sums) * nx * P >= ROW_BYTES;
+}
+
+// Bytes a node of the sums that a step of [n0, n0 + nsteps) adds to, on average.
+double span_sum_bytes(const LensEpi2D &e, int n0, int nsteps) {
+    auto met = [&](long a, long b) { return (double)std::max(0L, std::min(b, (long)n0 + nsteps) - std::max(a, (long)n0)); };
+    const double k = met(e.dft_n0, e.dft_n1) * ((e.dft ? 16 : 0) + (e.dft_ex ? 16 : 0)) +
+                     (e.dft_prev ? 16 * met(e.prev_n0, e.prev_n1) : 0.0) + (e.iavg ? 4 * met(e.iavg_n0, 1L << 40) : 0.0);
+    return k / std::max(nsteps, 1);
+}
+
+// TM spans that read a table: the passes are wide inside the windows too (the one-cell E pass reads
+// every row), where repeated rows leave the L2 to the sums.
+bool table_tm(double cells, int ny, double sums) {
+    const int cb = (ny + BX * WV - 1) / (BX * WV);
+    const double pad = (double)cb * BX * WV / ny;
+    return wide_tm(cells, ny) || (sums > 0.0 && cells >= 1.1e6 && pad <= 2.0 && (cb > 1 || pad <= 1.5));
 }
 
 int row_table(const RowArrays &v, int nx, int ny, int P, int *rowref, void *stream) {
@@ -958,17 +992,19 @@ int tm2d_run(const LensTM2D *g, const LensStepTable *tab, const LensEpi2D *ep, c
     const dim3 blk(BX, BY), grd((g->ny + BX - 1) / BX, (g->nx + BY - 1) / BY);
     const double cells = (double)g->nx * g->ny;
     const bool ok = wide_ok(e, dr, {g->ex, g->ey, g->hz, g->ca_x, g->ca_y, g->da_x, g->da_y}), wide = ok && wide_tm(cells, g->ny);
+    const double state = (double)g->nx * g->pitch;
     if (wide || (ok && cells >= TM_BOX)) {
         const dim3 wb(BX, WT), wg((g->ny + BX * WV - 1) / (BX * WV), (g->nx + WT * WR - 1) / (WT * WR)), bg = box_grid(e, g->nx, g->ny);
         for (int n = n0; n < n0 + nsteps; ++n) {
-            if (wide) {
+            const bool sums = epi2d_beyond_boxes(&e, n);
+            if (sums ? rowref || wide_tm_sums(cells, g->ny, state * (4 * (g->da_x ? 7 : 5) + sum_bytes(e, n))) : wide) {
                 go([&] { tm2d_h_wide<<<wg, wb, 0, s>>>(*g); });
                 go([&] { tm2d_e_wide<<<wg, wb, 0, s>>>(*g, rowref, *tab, n); });
             } else {
                 go([&] { tm2d_h<<<grd, blk, 0, s>>>(*g); });
                 go([&] { tm2d_e<<<grd, blk, 0, s>>>(*g, *tab, n, d); });
             }
-            if (epi2d_beyond_boxes(&e, n)) go([&] { tm2d_epi<<<grd, blk, 0, s>>>(*g, *tab, e, n); });
+            if (sums) go([&] { tm2d_epi<<<grd, blk, 0, s>>>(*g, *tab, e, n); });
             else if (bg.x > 0) go([&] { box2d<<<bg, blk, 0, s>>>(*g, e); });
         }
         return dry ? LENS_OK : lens_cuda_status();
@@ -1027,18 +1063,20 @@ extern "C" int lens_tm2d_step_launches(const LensTM2D *g, const LensStepTable *t
     return st == LENS_OK ? n : st;
 }
 
-extern "C" int lens_te2d_row_table(const LensTE2D *g, const LensEpi2D *ep, int nsteps, int *rowref, void *stream) {
+extern "C" int lens_te2d_row_table(const LensTE2D *g, const LensEpi2D *ep, int n0, int nsteps, int *rowref, void *stream) {
     if (!rowref) return LENS_ERR_ARG;
-    if (!grid2d_ok(g) || !g->ce_e || !g->ce_h || !row_table_pays(g->nx, g->pitch, 5, nsteps) ||
+    if (!grid2d_ok(g) || !g->ce_e || !g->ce_h || !row_table_pays(g->nx, g->pitch, 5, 0.0, nsteps) ||
         !wide_te((double)g->nx * g->ny, g->ny) || !wide_ok(ep ? *ep : empty_epi(), nullptr, {g->ez, g->hx, g->hy, g->ce_e, g->ce_h}))
         return LENS_ERR_SIZE;
+    if (ep && span_sum_bytes(*ep, n0, nsteps) >= 8.0) return LENS_ERR_SIZE;  // half of the steps or more read every row
     return row_table(RowArrays{{g->ce_e, g->ce_h}, {g->nx, g->nx}, 2}, g->nx, g->ny, g->pitch, rowref, stream);
 }
 
-extern "C" int lens_tm2d_row_table(const LensTM2D *g, const LensEpi2D *ep, int nsteps, int *rowref, void *stream) {
+extern "C" int lens_tm2d_row_table(const LensTM2D *g, const LensEpi2D *ep, int n0, int nsteps, int *rowref, void *stream) {
     if (!rowref) return LENS_ERR_ARG;
+    const double sums = ep && nsteps > 0 ? span_sum_bytes(*ep, n0, nsteps) : 0.0;
     if (!grid2d_ok(g) || !g->ca_x || !g->ca_y || (!g->da_x) != (!g->da_y) ||
-        !row_table_pays(g->nx, g->pitch, g->da_x ? 7 : 5, nsteps) || !wide_tm((double)g->nx * g->ny, g->ny) ||
+        !row_table_pays(g->nx, g->pitch, g->da_x ? 7 : 5, sums, nsteps) || !table_tm((double)g->nx * g->ny, g->ny, sums) ||
         !wide_ok(ep ? *ep : empty_epi(), nullptr, {g->ex, g->ey, g->hz, g->ca_x, g->ca_y, g->da_x, g->da_y}))
         return LENS_ERR_SIZE;
     return row_table(RowArrays{{g->ca_x, g->ca_y, g->da_x, g->da_y}, {g->nx - 1, g->nx, g->nx - 1, g->nx}, g->da_x ? 4 : 2},

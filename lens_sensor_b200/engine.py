@@ -314,20 +314,19 @@ class Grid2D:
                     self._made.value += 1
                     self.rs_stream = on
                     return N.check(st)
-            # (TE steps with sums read every row: their E pass is the one-cell one)
-            if self.rowref is not None and not (epi is not None and self.pol == 's' and sums_a_step(epi.s, n0, nsteps)):
-                rows = self._row_table(e, nsteps, stream)
+            if self.rowref is not None:
+                rows = self._row_table(e, n0, nsteps, stream)
         d = ctypes.byref(drive.s) if drive is not None else None
         N.check(self._step(ctypes.byref(self.s), rows, ctypes.byref(table.s), e, d, n0, nsteps, ctypes.byref(self._made),
                            _stream_ptr(stream)))
         if rows is not None:
             self._made.value += 2
 
-    def _row_table(self, e, nsteps, stream):
-        """The table of repeated coefficient rows for a span of nsteps, from the coefficients as
+    def _row_table(self, e, n0, nsteps, stream):
+        """The table of repeated coefficient rows for the span [n0, n0 + nsteps), from the coefficients as
         they are now (they may be written between calls in any way); None where the span would
         not gain by it."""
-        st = self._rows(ctypes.byref(self.s), e, nsteps, _ptr(self.rowref), _stream_ptr(stream))
+        st = self._rows(ctypes.byref(self.s), e, n0, nsteps, _ptr(self.rowref), _stream_ptr(stream))
         if st == N.ERR_SIZE:
             return None
         N.check(st)

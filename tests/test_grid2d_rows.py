@@ -47,14 +47,14 @@ def test_table_is_the_first_row_of_each_run(case):
     co[-1][11].view(torch.int32)[ny - 2] ^= 1  # one bit of one value
     ref = torch.full((nx,), -1, dtype=torch.int32, device='cuda')
     fn = g.lib.lens_te2d_row_table if pol == 's' else g.lib.lens_tm2d_row_table
-    assert fn(ctypes.byref(g.s), None, 1 << 20, E._ptr(ref), None) == 0
+    assert fn(ctypes.byref(g.s), None, 0, 1 << 20, E._ptr(ref), None) == 0
     want = E.repeated_rows(co)
     if pol == 'p':      # the last row has no Ex: Ey's coefficients alone decide
         want[nx - 1] = E.repeated_rows([c for c in co[1::2]])[nx - 1] if bool(
             all(torch.equal(c[nx - 1], c[nx - 2]) for c in co[1::2])) else nx - 1
     assert torch.equal(ref, want)
     assert ref[12] != ref[10] and int((ref == torch.arange(nx, device='cuda')).sum()) < nx
-    assert fn(ctypes.byref(g.s), None, 1, E._ptr(ref), None) == N.ERR_SIZE   # one step does not gain by it
+    assert fn(ctypes.byref(g.s), None, 0, 1, E._ptr(ref), None) == N.ERR_SIZE   # one step does not gain by it
 
 
 @pytest.mark.gpu
@@ -132,6 +132,28 @@ def test_wide_passes_without_a_table(case):
     _same(a, b)
     for q in ('dft', 'prev', 'iavg'):
         assert torch.equal(getattr(ea, q), getattr(eb, q)), q
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize('nx,ny', [(10001, 130), (6901, 200), (3701, 399)])
+def test_tm_windows_with_a_table(nx, ny):
+    """Grids whose fields lie in the L2 and, with their sums, beyond it: a table and wide passes inside the windows."""
+    import torch
+    a, b = (_grid('p', nx, ny, True, 9) for _ in range(2))
+    a.rs_scratch, a.rowref = None, torch.empty(nx, dtype=torch.int32, device='cuda')   # step by step
+    tab = _tab(a, 16)
+    ea, eb = _epi(a, 16, True), _epi(b, 16, True)
+    was = a.launches
+    a.step(tab, 7, 16, ea)
+    assert a.launches - was == 2 + 3 * 16
+    _one_cell(b, tab, 7, 16, eb)
+    torch.cuda.synchronize()
+    _same(a, b)
+    for q in ('dft', 'dft_ex', 'prev', 'iavg'):
+        assert torch.equal(getattr(ea, q), getattr(eb, q)), q
+    far = N.Epi2D.from_buffer_copy(ea.s)      # the same arrays, their windows elsewhere: nothing to gain
+    far.dft_n0, far.dft_n1, far.prev_n0, far.prev_n1, far.iavg_n0 = 90, 99, 90, 99, 90
+    assert a.lib.lens_tm2d_row_table(ctypes.byref(a.s), ctypes.byref(far), 7, 16, a.rowref.data_ptr(), None) == N.ERR_SIZE
 
 
 @pytest.mark.gpu

@@ -39,7 +39,7 @@ def _epi(box=False, dft=None):
 
 @pytest.mark.parametrize('pol,nx,ny,plain,box,window', [
     ('s', 140, 96, 2, 2, 2), ('p', 140, 96, 2, 3, 3),           # one cell a thread; TM's epilogue is a launch
-    ('s', 3000, 400, 2, 2, 2), ('s', 3500, 400, 2, 3, 2),       # wide: boxes are a launch, small ones from 1.3 M cells;
+    ('s', 2900, 400, 2, 2, 2), ('s', 3500, 400, 2, 3, 2),       # wide: boxes are a launch, small ones from 1.2 M cells;
     ('s', 8000, 300, 2, 3, 2), ('p', 4000, 200, 2, 3, 3)])      # TE sums with the E pass that holds the field
 def test_launches_of_a_step(pol, nx, ny, plain, box, window):
     assert _count(pol, nx, ny) == 10 * plain
