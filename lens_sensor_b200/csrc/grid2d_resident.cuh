@@ -31,7 +31,7 @@
 // warps at the y faces, about 0.1 us a row.  The step by step launches (two or three a
 // step, one cell a thread) took 8.2 us a step on 140 x 96 cells (launches), 18.3 on 1600 x
 // 480 (L2 latency) and 27.7 on 1201 x 431 absorbing TM cells with every epilogue on; this
-// kernel takes 1.35, 3.3 and 13.7 (the last bound by the compensated sums' traffic in L2
+// kernel takes 1.5, 3.3 and 13.4 (the last bound by the compensated sums' traffic in L2
 // and shared memory: 16 bytes a node and DFT, read and written each step).
 // A row is instantiated in four forms, each warp taking the least that its rows and
 // columns need:
