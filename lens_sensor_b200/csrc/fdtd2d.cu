@@ -317,10 +317,10 @@ __global__ void __launch_bounds__(BX *BY)
 // coefficients, whose rows a layered grid repeats: rowref names the row to read, so a
 // repeated row comes from the caches (NULL: every row its own).  Memory latency bounds
 // them: 16000 x 700 cells with boxes, us a step TM / TE: 298 / 290 at one cell a thread (the
-// kernels above, kept for the forms only they carry), 106 / 95 here with 32 warps an SM, 110 /
-// 98 in blocks of 8 warps, 139 / 122 without the register cap, 137 / 111 with 3 rows, 125 / 112
-// with one row and 48 warps.  Warps clear of strips, faces and source rows run without tests
-// (without that form: 178 / 165).
+// kernels above, kept for the forms and sizes that the rules below leave to them), 106 / 95 here
+// with 32 warps an SM, 110 / 98 in blocks of 8 warps, 139 / 122 without the register cap, 137 / 111
+// with 3 rows, 125 / 112 with one row and 48 warps.  Warps clear of strips, faces and source rows run
+// without tests (without that form: 178 / 165).
 // The multiply-adds are written out and round as those kernels do, and as
 // grid2d_resident.cuh.
 constexpr int WV = 4, WR = 2, WT = 4;   // columns, rows of a thread; warps of a block (along x)
